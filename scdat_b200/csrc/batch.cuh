@@ -78,10 +78,11 @@ struct BlockMap {
     int blocks;
 };
 
-// push (push_mixed.cu); chunk_prefix[j] = first 32-particle chunk of job j, computed on the
-// device from the live counts by launch_batch_prefix, which also zeroes the pass's work counter
-// ctr[pass - 1].
-void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int64_t* chunk_prefix, unsigned* ctr,
+// push (push_mixed.cu); chunk_prefix[j] = first work unit of job j (njobs + 2 entries: the total
+// and the 32-particle chunks per unit follow the jobs), computed on the device from the live
+// counts by launch_batch_prefix for a pass of `grid` blocks, which also zeroes the pass's work
+// counter ctr[pass - 1].
+void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int grid, int64_t* chunk_prefix, unsigned* ctr,
                          cudaStream_t st);
 void launch_push_mixed_batch(const PushJob* jobs, int njobs, const int64_t* chunk_prefix, unsigned* ctr, int pass,
                              int grid, cudaStream_t st);

@@ -208,7 +208,7 @@ void enqueue_front(scdat_batch* b, cudaStream_t s)
     launch_batch_zero(b->fjobs.p, b->pjobs.p, nc, nj, b->nsm * 2, s);
     const int grid = b->nsm * b->tune.push_blocks_per_sm;
     for (int pass = 1; pass <= 3; ++pass) {
-        launch_batch_prefix(b->pjobs.p, nj, pass, b->prefix.p, b->pass_ctr.p, s);
+        launch_batch_prefix(b->pjobs.p, nj, pass, grid, b->prefix.p, b->pass_ctr.p, s);
         launch_push_mixed_batch(b->pjobs.p, nj, b->prefix.p, b->pass_ctr.p, pass, grid, s);
     }
     launch_batch_surface(b->fjobs.p, nc, s);
@@ -407,7 +407,7 @@ SCDAT_API int scdat_batch_create(int32_t n, scdat_ctx* const* ctxs, scdat_batch*
     BCK(b->dcount.alloc(2 * (size_t)njobs));
     BCK(b->pjobs.alloc((size_t)njobs));
     BCK(b->fjobs.alloc((size_t)n));
-    BCK(b->prefix.alloc((size_t)njobs + 1));
+    BCK(b->prefix.alloc((size_t)njobs + 2));
     BCK(b->pass_ctr.alloc(3));
     BCK(b->sco.alloc((size_t)n));
     BCK(cudaMemsetAsync(b->sco.p, 0, sizeof(PcgScalars) * n, b->st));

@@ -276,6 +276,8 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
             P.id = Ss.id2.p;
         }
         SpeciesDev sd = species_dev(ctx, s);
+        // no more blocks than the species has chunks for (8 warps a block, a chunk each), but one per SM
+        const int grid = (int)std::max<int64_t>(ctx->nsm, std::min<int64_t>(ctx->grid_push, (Ss.n + 255) / 256));
         // defer-list counts [0, 1] and the three passes' work counters [2, 5)
         CK(cudaMemsetAsync(ctx->dcount.p, 0, 5 * sizeof(unsigned), ctx->st));
         DeferList d1{ctx->dcount.p, ctx->d1cap, ctx->d1idx.p, ctx->d1it.p, ctx->d1rem.p, ctx->d1vs.p};
@@ -286,7 +288,7 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         if (ctx->mixed) {
             const bool stay = stay_first_now(ctx, s);
             launch_push_mixed(ctx->mv, P, R, sd, pp, d1, d2, acc, ctx->led.p, ctx->ke_acc.p, ctx->dcount.p + 2,
-                              ctx->grid_push, stay, ctx->st);
+                              grid, stay, ctx->st);
             if (Ss.perm_pending) {
                 Ss.perm_pending = false;
                 Ss.mix.swap(Ss.mix2);
@@ -302,7 +304,7 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
             }
         } else
             launch_push_f64(ctx->mv, P, sd, pp, d1, d2, acc, ctx->led.p, ctx->ke_acc.p, ctx->dcount.p + 2,
-                            ctx->grid_push, ctx->st);
+                            grid, ctx->st);
     }
     CK(cudaGetLastError());
     if (ctx->timing) {

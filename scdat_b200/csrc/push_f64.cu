@@ -209,12 +209,13 @@ __global__ void __launch_bounds__(256) k_push_f64(const __grid_constant__ MeshVi
     const int64_t n = *P.count;
     PushStats c{0.0, 0u, 0u};
     const int lane = threadIdx.x & 31;
+    const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
     warp_stats_begin();
     for (;;) {
-        // runs of kRun chunks, as in the mixed form
-        const int64_t b0 = (int64_t)next_chunk(ctr) * (32 * kRun);
+        // runs of chunks, as in the mixed form
+        const int64_t b0 = (int64_t)next_chunk(ctr) * run;
         if (b0 >= n) break;
-        for (int64_t base = b0; base < b0 + 32 * kRun && base < n; base += 32) {
+        for (int64_t base = b0; base < b0 + run && base < n; base += 32) {
             const int64_t i = base + lane;
             int st = -1;
             FlightD f;

@@ -580,7 +580,7 @@ __device__ __forceinline__ void push_more_warp(const MeshView& M, const Particle
     warp_chunk_end(c);
 }
 
-// Pass 1: every stored particle.  Warps take runs of kRun 32-particle chunks from the launch's
+// Pass 1: every stored particle.  Warps take runs of 32-particle chunks from the launch's
 // work counter until none are left, so no warp idles while another still has work.
 // 5 blocks of 256 per SM (48 registers): with the record's vector loads and the folded re-sort
 // gather, the fewer spills now pay more than the sixth block's warps (push per step at 128^3:
@@ -594,11 +594,12 @@ __global__ void __launch_bounds__(256, 5) k_push_mixed(const __grid_constant__ M
 {
     const int64_t n = *P.count;
     PushStats c{0.0, 0u, 0u};
+    const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
     warp_stats_begin();
     for (;;) {
-        const int64_t b0 = (int64_t)next_chunk(ctr) * (32 * kRun);
+        const int64_t b0 = (int64_t)next_chunk(ctr) * run;
         if (b0 >= n) break;
-        for (int64_t base = b0; base < b0 + 32 * kRun && base < n; base += 32)
+        for (int64_t base = b0; base < b0 + run && base < n; base += 32)
             push1_warp(M, P, R, S, pp, D, A, L, base, n, c);
     }
     warp_stats_flush(L, ke_acc, S.vmax);
@@ -618,11 +619,12 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_stay(const __grid_constan
 {
     const int64_t n = *P.count;
     PushStats c{0.0, 0u, 0u};
+    const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
     warp_stats_begin();
     for (;;) {
-        const int64_t b0 = (int64_t)next_chunk(ctr) * (32 * kRun);
+        const int64_t b0 = (int64_t)next_chunk(ctr) * run;
         if (b0 >= n) break;
-        for (int64_t base = b0; base < b0 + 32 * kRun && base < n; base += 32)
+        for (int64_t base = b0; base < b0 + run && base < n; base += 32)
             push1_stay_warp(M, P, R, S, pp, D, A, L, base, n, c);
     }
     warp_stats_flush(L, ke_acc, S.vmax);
@@ -648,8 +650,10 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_more(const __grid_constan
 }
 
 // ---- batched step: all (scenario, species) jobs in one launch per pass -----------------
-__global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int pass, int64_t* __restrict__ pre,
-                               unsigned* __restrict__ ctr)
+// pre[njobs + 1]: 32-particle chunks per unit, chosen over all jobs (run_chunks; warps: those of
+// the pass's launch).
+__global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int pass, int64_t warps,
+                               int64_t* __restrict__ pre, unsigned* __restrict__ ctr)
 {
     __shared__ int64_t cnt[kMaxBatchJobs];
     for (int j = threadIdx.x; j < njobs; j += blockDim.x) {
@@ -661,23 +665,27 @@ __global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int 
             n = min((int64_t)*J.D1.count, (int64_t)J.D1.cap);
         else
             n = min((int64_t)*J.D2.count, (int64_t)J.D2.cap);
-        const int64_t unit = pass == 1 ? 32 * kRun : 32;  // particles per counter value
-        cnt[j] = (n + unit - 1) / unit;
+        cnt[j] = n;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        int64_t total = 0;
+        for (int j = 0; j < njobs; ++j) total += cnt[j];
+        const int run = pass == 1 ? run_chunks(total, warps) : 1;
+        const int64_t unit = 32 * run;  // particles per counter value
         int64_t a = 0;
         for (int j = 0; j < njobs; ++j) {
             pre[j] = a;
-            a += cnt[j];
+            a += (cnt[j] + unit - 1) / unit;
         }
         pre[njobs] = a;
+        pre[njobs + 1] = run;
         ctr[pass - 1] = 0u;
     }
 }
 
 // Pass `pass` (1, 2 or 3) of every job.  Warps take units g of the global index from the pass's
-// work counter (pass 1: runs of kRun 32-particle chunks; passes 2 and 3: single chunks); unit g
+// work counter (pass 1: runs of pre[njobs + 1] 32-particle chunks; passes 2 and 3: single chunks); unit g
 // belongs to the job j with pre[j] <= g < pre[j + 1], and a warp flushes its statistics into a
 // job's ledger when it moves on to another job.
 template <int PASS>
@@ -688,6 +696,7 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __re
     for (int j = threadIdx.x; j <= njobs; j += blockDim.x) spre[j] = pre[j];
     __syncthreads();
     const int64_t total = spre[njobs];
+    const int64_t run = PASS == 1 ? 32 * pre[njobs + 1] : 32;
     PushStats c{0.0, 0u, 0u};
     warp_stats_begin();
     int cur = -1;
@@ -708,8 +717,8 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __re
         }
         const PushJob& J = jobs[cur];
         if (PASS == 1) {
-            const int64_t n = *J.P.count, b0 = (g - spre[cur]) * (32 * kRun);
-            for (int64_t base = b0; base < b0 + 32 * kRun && base < n; base += 32)
+            const int64_t n = *J.P.count, b0 = (g - spre[cur]) * run;
+            for (int64_t base = b0; base < b0 + run && base < n; base += 32)
                 push1_warp(J.M, J.P, SortedSource{}, J.S, J.pp, J.D1, J.A, J.L, base, n, c);
             continue;
         }
@@ -824,10 +833,10 @@ void launch_from_mixed(const MeshView& M, int64_t n, const ParticleStore& P, dou
     k_from_mixed<<<148 * 4, 256, 0, st>>>(M, n, P, x, y, z, vx, vy, vz);
 }
 
-void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int64_t* chunk_prefix, unsigned* ctr,
+void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int grid, int64_t* chunk_prefix, unsigned* ctr,
                          cudaStream_t st)
 {
-    k_batch_prefix<<<1, 1024, 0, st>>>(jobs, njobs, pass, chunk_prefix, ctr);
+    k_batch_prefix<<<1, 1024, 0, st>>>(jobs, njobs, pass, 8ll * grid, chunk_prefix, ctr);
 }
 
 void launch_push_mixed_batch(const PushJob* jobs, int njobs, const int64_t* chunk_prefix, unsigned* ctr, int pass,
