@@ -69,39 +69,6 @@ __device__ __forceinline__ bool bary64(const MeshView& M, int t, double px, doub
     return bary_inside(lam);
 }
 
-// Lowest-id tet containing p among the grid candidates (exactly the result of the
-// reference's linear scan, PICParticleAlgorithms.cpp:882-888), or -1.
-static __device__ __noinline__ int grid_lookup(const MeshView& M, double px, double py, double pz)
-{
-    double p[3] = {px, py, pz};
-    int lo[3], hi[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        double l = (p[a] - M.gdelta - M.gmin[a]) * M.ginv[a];
-        double h = (p[a] + M.gdelta - M.gmin[a]) * M.ginv[a];
-        if (!(h >= 0.0) || !(l < (double)M.gdim[a])) return -1;  // outside the grid (or NaN)
-        lo[a] = l < 0.0 ? 0 : (int)l;
-        hi[a] = h >= (double)M.gdim[a] ? M.gdim[a] - 1 : (int)h;
-    }
-    int best = 0x7fffffff;
-    double lam[4];
-    for (int k = lo[2]; k <= hi[2]; ++k)
-        for (int j = lo[1]; j <= hi[1]; ++j)
-            for (int i = lo[0]; i <= hi[0]; ++i) {
-                int b = i + M.gdim[0] * (j + M.gdim[1] * k);
-                int s = __ldg(M.bin_start + b), e = __ldg(M.bin_start + b + 1);
-                for (int q = s; q < e; ++q) {
-                    int t = __ldg(M.bin_tets + q);
-                    if (t >= best) break;
-                    if (bary64(M, t, px, py, pz, lam)) {
-                        best = t;
-                        break;
-                    }
-                }
-            }
-    return best == 0x7fffffff ? -1 : best;
-}
-
 __device__ __forceinline__ int4 rec_nbr(const MeshView& M, int t)
 {
     return __ldg(reinterpret_cast<const int4*>(M.geom + 16 * (int64_t)t + 12));
@@ -142,10 +109,81 @@ __device__ __forceinline__ int walk64(const MeshView& M, double px, double py, d
     return -1;
 }
 
+// p lies outside the locate grid widened by the containment tolerance (or is NaN): no tet holds it.
+__device__ __forceinline__ bool outside_grid(const MeshView& M, double px, double py, double pz)
+{
+    const double p[3] = {px, py, pz};
+    bool out = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double l = (p[a] - M.gdelta - M.gmin[a]) * M.ginv[a];
+        const double h = (p[a] + M.gdelta - M.gmin[a]) * M.ginv[a];
+        out = out || !(h >= 0.0) || !(l < (double)M.gdim[a]);
+    }
+    return out;
+}
+
+// Lowest-id tet containing p among the grid candidates (exactly the result of the
+// reference's linear scan, PICParticleAlgorithms.cpp:882-888), or -1.
+static __device__ __noinline__ int grid_lookup(const MeshView& M, double px, double py, double pz)
+{
+    if (outside_grid(M, px, py, pz)) return -1;
+    double p[3] = {px, py, pz};
+    int lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        double l = (p[a] - M.gdelta - M.gmin[a]) * M.ginv[a];
+        double h = (p[a] + M.gdelta - M.gmin[a]) * M.ginv[a];
+        lo[a] = l < 0.0 ? 0 : (int)l;
+        hi[a] = h >= (double)M.gdim[a] ? M.gdim[a] - 1 : (int)h;
+    }
+    int best = 0x7fffffff;
+    double lam[4];
+    for (int k = lo[2]; k <= hi[2]; ++k)
+        for (int j = lo[1]; j <= hi[1]; ++j)
+            for (int i = lo[0]; i <= hi[0]; ++i) {
+                int b = i + M.gdim[0] * (j + M.gdim[1] * k);
+                int s = __ldg(M.bin_start + b), e = __ldg(M.bin_start + b + 1);
+                for (int q = s; q < e; ++q) {
+                    int t = __ldg(M.bin_tets + q);
+                    if (t >= best) break;
+                    if (bary64(M, t, px, py, pz, lam)) {
+                        best = t;
+                        break;
+                    }
+                }
+            }
+    return best == 0x7fffffff ? -1 : best;
+}
+
+// The unique tet holding p, by a walk from the last tet of p's grid bin (a few steps away at
+// most, where a scan of the bin tests every candidate below the holder's id); -1 when p is in no
+// tet, or in the tolerance band of several, or the walk cannot decide.  p is inside the grid.
+__device__ __forceinline__ int walk_from_bin(const MeshView& M, double px, double py, double pz)
+{
+    const double p[3] = {px, py, pz};
+    int b = 0, mul = 1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int c = (int)((p[a] - M.gmin[a]) * M.ginv[a]);
+        b += mul * (c < 0 ? 0 : (c >= M.gdim[a] ? M.gdim[a] - 1 : c));
+        mul *= M.gdim[a];
+    }
+    const int e = __ldg(M.bin_start + b + 1);
+    if (e == __ldg(M.bin_start + b)) return -1;
+    const int t0 = __ldg(M.bin_tets + e - 1);
+    double lam[4];
+    bool uniq = false;
+    bary64(M, t0, px, py, pz, lam);
+    const int t = walk64(M, px, py, pz, t0, lam, &uniq);
+    return uniq ? t : -1;
+}
+
 // Without a usable hint: walk from `start` when given, else (or when the walk cannot decide)
 // the exact grid lookup of the lowest containing id.
 static __device__ __noinline__ int locate_far(const MeshView& M, double px, double py, double pz, int start)
 {
+    if (outside_grid(M, px, py, pz)) return -1;  // most calls: a particle that left the domain
     if (start >= 0) {
         double lam[4];
         bary64(M, start, px, py, pz, lam);
@@ -163,6 +201,7 @@ static __device__ __noinline__ int locate_far(const MeshView& M, double px, doub
 static __device__ __noinline__ int locate_slow(const MeshView& M, double px, double py, double pz, int hint,
                                                double lam[4])
 {
+    if (outside_grid(M, px, py, pz)) return -1;  // then neither the walk nor the lists can find it
     bool uniq = false;
     int t = walk64(M, px, py, pz, hint, lam, &uniq);
     if (t >= 0 && uniq) return t;
@@ -185,6 +224,16 @@ __device__ __forceinline__ int locate(const MeshView& M, double px, double py, d
         return locate_slow(M, px, py, pz, hint, lam);
     }
     return grid_lookup(M, px, py, pz);
+}
+
+// locate() for a point far from its hint (a periodic image, usually across the whole box, which a
+// walk from the hint cannot reach in its step cap): the walk from the point's bin first.  A unique
+// holder is what every search order finds, so the result is locate()'s.
+__device__ __forceinline__ int locate_image(const MeshView& M, double px, double py, double pz, int hint)
+{
+    if (outside_grid(M, px, py, pz)) return -1;
+    const int t = walk_from_bin(M, px, py, pz);
+    return t >= 0 ? t : locate(M, px, py, pz, hint);
 }
 
 // PICCycle::detectBoundaryFace, PICCycle.cpp:1074-1133.
@@ -306,7 +355,7 @@ static __device__ __noinline__ int resolve_lost(const MeshView& M, const Species
             if (c[a] < 0.0) c[a] += Lp;
         }
         px = c[0]; py = c[1]; pz = c[2];
-        int h2 = locate(M, px, py, pz, hint);
+        int h2 = locate_image(M, px, py, pz, hint);
         hint = h2;
         if (h2 >= 0) resolved = h2;
     }
