@@ -10,6 +10,7 @@
 #pragma once
 
 #include "field.cuh"
+#include "pcg_group.cuh"
 #include "push.cuh"
 #include "surface.cuh"
 
@@ -47,6 +48,7 @@ struct FieldJob {
     double sign;
     double *b, *x, *r;
     float *rf, *xf, *zf, *pf, *pnf, *qf, *qq;
+    double* zp;       // [2 R] of the one-launch solve
     PcgScalars* sc;   // inner (FP32) solve
     PcgScalars* sco;  // outer refinement loop
     double* part;
@@ -94,6 +96,9 @@ void launch_batch_zero(const FieldJob* jobs, const PushJob* pjobs, int njobs, in
 void launch_batch_surface(const FieldJob* jobs, int njobs, cudaStream_t st);
 void launch_batch_finalize_rhs(const FieldJob* jobs, const BlockMap& nodes, const BlockMap& rows, cudaStream_t st);
 void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const BlockMap& rows, int njobs, cudaStream_t st);
+// the mixed solve of all scenarios as one launch, when cg_plan found room for their groups
+cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const CgPlan& plan, cudaStream_t st);
+// otherwise as two nested loops of launches:
 void launch_batch_outer_begin(const FieldJob* jobs, const BlockMap& rows, int njobs, unsigned long long cond_inner,
                               int* any_out, cudaStream_t st);
 // passes[0] counts refinement passes, passes[1] inner double-iterations (launch accounting)

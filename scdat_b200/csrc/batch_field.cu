@@ -5,6 +5,7 @@
 // convergence flags, and CUDA-graph conditional handles when the step is captured).
 #include "batch.cuh"
 #include "field_kern.cuh"
+#include "pcg_group.cuh"
 
 namespace scdat {
 
@@ -84,10 +85,13 @@ __global__ void k_batch_rhs(const FieldJob* __restrict__ jobs, BlockMap m)
     k_rhs_body(J.A, J.rho, J.phi, J.sign, J.b, g);
 }
 
-// one thread per scenario: a fresh refinement loop
-__global__ void k_batch_prologue(const FieldJob* __restrict__ jobs, int njobs)
+// one block per scenario: a fresh refinement loop, and zero barrier slots for the one-launch solve
+__global__ void k_batch_prologue(const FieldJob* __restrict__ jobs)
 {
-    for (int k = threadIdx.x; k < njobs; k += blockDim.x) {
+    const int k = blockIdx.x;
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(jobs[k].part);
+    for (size_t i = threadIdx.x; i < kCgSlotBytes / sizeof(*slots); i += blockDim.x) slots[i] = 0ull;
+    if (threadIdx.x == 0) {
         PcgScalars* o = jobs[k].sco;
         o->iter = 0;
         o->outer = 0;  // outer iterations
@@ -95,6 +99,19 @@ __global__ void k_batch_prologue(const FieldJob* __restrict__ jobs, int njobs)
         o->rtol = jobs[k].rtol;
         o->max_iter = jobs[k].max_iter;
     }
+}
+
+// The whole mixed solve of every scenario in one cooperative launch (pcg_group.cuh): the blocks
+// m gives a scenario are its group, and no group waits for another.
+template <int KR>
+__global__ void __launch_bounds__(kCgMaxThreads, 1) k_batch_solve(const FieldJob* __restrict__ jobs, BlockMap m, int smem_bytes)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    Grid gr;
+    const FieldJob& J = jobs[map_ctx(m, gr)];
+    if (J.A.R == 0) return;
+    CgGroup g{gr.b, gr.n, reinterpret_cast<unsigned long long*>(J.part)};
+    cg_solve_mixed<KR>(g, J.A, J.b, J.x, reinterpret_cast<double2*>(J.zp), J.sco, J.rtol, J.max_iter, smem, smem_bytes);
 }
 
 // FP64 residual r = b - A x and its norms into the outer scalars
@@ -261,7 +278,22 @@ void launch_batch_finalize_rhs(const FieldJob* jobs, const BlockMap& nodes, cons
 
 void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const BlockMap&, int njobs, cudaStream_t st)
 {
-    k_batch_prologue<<<1, 256, 0, st>>>(jobs, njobs);
+    k_batch_prologue<<<njobs, 256, 0, st>>>(jobs);
+}
+
+cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const CgPlan& plan, cudaStream_t st)
+{
+    auto kernel = plan.rows_per_thread == 1   ? k_batch_solve<1>
+                  : plan.rows_per_thread == 2 ? k_batch_solve<2>
+                  : plan.rows_per_thread == 3 ? k_batch_solve<3>
+                                              : k_batch_solve<4>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemBytes);
+    if (e != cudaSuccess) return e;
+    BlockMap m = groups;
+    int smem = plan.smem;
+    void* args[] = {&jobs, &m, &smem};
+    return cudaLaunchCooperativeKernel((const void*)kernel, dim3(plan.blocks), dim3(plan.threads), args,
+                                       (size_t)plan.smem, st);
 }
 
 void launch_batch_outer_begin(const FieldJob* jobs, const BlockMap& rows, int njobs, unsigned long long cond_inner,

@@ -29,23 +29,32 @@ struct MapBufs {
     BlockMap view{};
 };
 
+int upload_map(MapBufs& m, const std::vector<int>& blocks, cudaStream_t st)
+{
+    const int n = (int)blocks.size();
+    std::vector<int> first((size_t)n + 1, 0), of;
+    for (int k = 0; k < n; ++k) {
+        first[k + 1] = first[k] + blocks[k];
+        for (int i = 0; i < blocks[k]; ++i) of.push_back(k);
+    }
+    if (m.ctx_of.upload(of.data(), of.size(), st) != cudaSuccess) return SCDAT_ERR_CUDA;
+    if (m.first.upload(first.data(), first.size(), st) != cudaSuccess) return SCDAT_ERR_CUDA;
+    m.view = BlockMap{m.ctx_of.p, m.first.p, first[n]};
+    return SCDAT_OK;
+}
+
 // Blocks per scenario in proportion to its share of `sizes` (at least one each).
 int build_map(MapBufs& m, const std::vector<int64_t>& sizes, int target, cudaStream_t st)
 {
     const int n = (int)sizes.size();
     double tot = 0.0;
     for (int64_t v : sizes) tot += (double)std::max<int64_t>(v, 1);
-    std::vector<int> first((size_t)n + 1, 0), of;
+    std::vector<int> blocks((size_t)n);
     for (int k = 0; k < n; ++k) {
         int b = (int)std::floor((double)target * (double)std::max<int64_t>(sizes[k], 1) / tot + 0.5);
-        b = std::max(1, std::min(b, target));
-        first[k + 1] = first[k] + b;
-        for (int i = 0; i < b; ++i) of.push_back(k);
+        blocks[k] = std::max(1, std::min(b, target));
     }
-    if (m.ctx_of.upload(of.data(), of.size(), st) != cudaSuccess) return SCDAT_ERR_CUDA;
-    if (m.first.upload(first.data(), first.size(), st) != cudaSuccess) return SCDAT_ERR_CUDA;
-    m.view = BlockMap{m.ctx_of.p, m.first.p, first[n]};
-    return SCDAT_OK;
+    return upload_map(m, blocks, st);
 }
 
 }  // namespace
@@ -65,6 +74,8 @@ struct scdat_batch {
     DBuf<unsigned long long> passes;  // [outer passes, inner double-iterations]
     int* any_host = nullptr;
     MapBufs nodes, rows, tets;
+    MapBufs groups;  // blocks of the one-launch solve, when it has room (solve.ok)
+    CgPlan solve;
     scdat_batch_tuning tune{};
     int nsm = 148;
     cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;
@@ -159,6 +170,7 @@ int upload_jobs(scdat_batch* b)
         F.pnf = c->pnf.p;
         F.qf = c->qf.p;
         F.qq = reinterpret_cast<float*>(c->q.p);
+        F.zp = c->p.p;
         F.sc = c->sc.p;
         F.sco = b->sco.p + k;
         F.part = c->part.p;
@@ -196,13 +208,18 @@ int build_maps(scdat_batch* b)
     int rc = build_map(b->nodes, nn, b->nsm * b->tune.field_blocks_per_sm, b->st);
     if (!rc) rc = build_map(b->rows, rr, b->nsm * b->tune.field_blocks_per_sm, b->st);
     if (!rc) rc = build_map(b->tets, tt, b->nsm * b->tune.field_blocks_per_sm, b->st);
+    if (!rc) {
+        std::vector<int> r(rr.begin(), rr.end()), blocks(rr.size());
+        b->solve = cg_plan(r.data(), (int)r.size(), b->nsm, blocks.data());
+        if (b->solve.ok) rc = upload_map(b->groups, blocks, b->st);
+    }
     if (rc) b->err = "block map upload failed";
     return rc;
 }
 
 // The step as launches on stream s.  With graph handles (cond_outer/cond_inner != 0) the
 // loops are conditional nodes added by the caller; without them the host drives the loops.
-void enqueue_front(scdat_batch* b, cudaStream_t s)
+int enqueue_front(scdat_batch* b, cudaStream_t s)
 {
     const int nj = (int)b->job_of.size(), nc = (int)b->ctx.size();
     launch_batch_zero(b->fjobs.p, b->pjobs.p, nc, nj, b->nsm * 2, s);
@@ -214,6 +231,8 @@ void enqueue_front(scdat_batch* b, cudaStream_t s)
     launch_batch_surface(b->fjobs.p, nc, s);
     launch_batch_finalize_rhs(b->fjobs.p, b->nodes.view, b->rows.view, s);
     launch_batch_pcg_mixed_prologue(b->fjobs.p, b->rows.view, nc, s);
+    if (b->solve.ok) BCK(launch_batch_solve(b->fjobs.p, b->groups.view, b->solve, s));
+    return SCDAT_OK;
 }
 
 void enqueue_back(scdat_batch* b, cudaStream_t s)
@@ -232,8 +251,9 @@ int read_any(scdat_batch* b)
 int step_eager(scdat_batch* b)
 {
     const int nc = (int)b->ctx.size();
-    enqueue_front(b, b->st);
-    for (int outer = 0; outer < 13; ++outer) {
+    int rc = enqueue_front(b, b->st);
+    if (rc) return rc;
+    for (int outer = 0; outer < 13 && !b->solve.ok; ++outer) {
         launch_batch_outer_begin(b->fjobs.p, b->rows.view, nc, 0ull, b->any.p, b->st);
         int a = read_any(b);
         if (a < 0) return SCDAT_ERR_CUDA;
@@ -277,14 +297,22 @@ int capture_graph(scdat_batch* b)
     b->release_graph();
     const int nc = (int)b->ctx.size();
     BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
-    enqueue_front(b, b->st);
+    int rc = enqueue_front(b, b->st);
+    if (rc) return rc;
+    if (b->solve.ok) {
+        enqueue_back(b, b->st);
+        BCK(cudaStreamEndCapture(b->st, &b->graph));
+        BCK(cudaGraphInstantiate(&b->exec, b->graph, 0));
+        b->graph_ready = true;
+        return SCDAT_OK;
+    }
     cudaStreamCaptureStatus cs;
     cudaGraph_t top = nullptr;
     BCK(cudaStreamGetCaptureInfo(b->st, &cs, nullptr, &top, nullptr, nullptr));
     cudaGraphConditionalHandle h_out;
     BCK(cudaGraphConditionalHandleCreate(&h_out, top, 1, cudaGraphCondAssignDefault));
     cudaGraph_t obody = nullptr;
-    int rc = add_while(b, b->st, h_out, &obody);
+    rc = add_while(b, b->st, h_out, &obody);
     if (rc) return rc;
     {
         BCK(cudaStreamBeginCaptureToGraph(b->st2, obody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
@@ -322,6 +350,10 @@ int after_steps(scdat_batch* b, int n)
     bool resorted = false;
     for (size_t k = 0; k < b->ctx.size(); ++k) {
         scdat_ctx* c = b->ctx[k];
+        if (o[k].done < 0) {
+            b->err = "field solve: a barrier wait ran out";
+            return SCDAT_ERR_CUDA;
+        }
         c->last_pcg_iter = o[k].iter;
         c->last_pcg_rel = std::sqrt(o[k].rr / (o[k].bb > 0.0 ? o[k].bb : 1.0));
         const int64_t before = c->steps;
@@ -526,14 +558,15 @@ SCDAT_API int scdat_batch_stream(const scdat_batch* b, void** stream)
     return SCDAT_OK;
 }
 
-// Kernels of this library launched by the steps so far: 16 per step plus 6 per refinement
-// pass and 5 per inner double-iteration (the loop passes are counted on the device).
+// Kernels of this library launched by the steps so far: 17 per step with the one-launch solve,
+// otherwise 16 plus 6 per refinement pass and 5 per inner double-iteration (the loop passes are
+// counted on the device).
 SCDAT_API int scdat_batch_kernel_launches(scdat_batch* b, int64_t* launches)
 {
     if (!b || !launches) return SCDAT_ERR_ARG;
     unsigned long long p[2] = {0, 0};
     BCK(cudaMemcpy(p, b->passes.p, sizeof(p), cudaMemcpyDeviceToHost));
-    *launches = 16 * b->steps + 6 * (int64_t)p[0] + 5 * (int64_t)p[1];
+    *launches = (b->solve.ok ? 17 : 16) * b->steps + 6 * (int64_t)p[0] + 5 * (int64_t)p[1];
     return SCDAT_OK;
 }
 

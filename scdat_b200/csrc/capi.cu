@@ -8,6 +8,7 @@
 // background MCC step of the reference driver (Main/main_PICcore.cpp:487-515).
 #include "ctx.cuh"
 #include "mg_setup.h"
+#include "pcg_group.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -387,6 +388,18 @@ int run_mgpcg(scdat_ctx* ctx, const V* b, V* x, V* r, V* z, V* p, V* q, double r
     return SCDAT_OK;
 }
 
+// The scalars of a one-launch solve, which marks them when a barrier wait ran out.
+int read_group_scalars(scdat_ctx* ctx, PcgScalars& h)
+{
+    int rc = read_scalars(ctx, h);
+    if (rc) return rc;
+    if (h.done < 0) {
+        ctx->err = "field solve: a barrier wait ran out";
+        return SCDAT_ERR_CUDA;
+    }
+    return SCDAT_OK;
+}
+
 int run_pcg64(scdat_ctx* ctx, const double* bvec, double* xvec, double rtol, int max_iter, int& iters,
               double& relres)
 {
@@ -394,6 +407,18 @@ int run_pcg64(scdat_ctx* ctx, const double* bvec, double* xvec, double rtol, int
     if (ctx->precond == SCDAT_PRECOND_MULTIGRID) {
         PcgScalars h{};
         int rc = run_mgpcg<double>(ctx, bvec, xvec, ctx->r.p, ctx->z.p, ctx->p.p, ctx->q.p, rtol, max_iter, h);
+        if (rc) return rc;
+        iters = h.iter;
+        relres = std::sqrt(h.rr / (h.bb > 0.0 ? h.bb : 1.0));
+        return SCDAT_OK;
+    }
+    int blocks;
+    const CgPlan plan = cg_plan(&A.R, 1, ctx->nsm, &blocks);
+    if (plan.ok) {
+        ++ctx->launches;
+        CK(launch_cg64(plan, A, bvec, xvec, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
+        PcgScalars h{};
+        int rc = read_group_scalars(ctx, h);
         if (rc) return rc;
         iters = h.iter;
         relres = std::sqrt(h.rr / (h.bb > 0.0 ? h.bb : 1.0));
@@ -436,6 +461,17 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
     iters = 0;
     relres = 0.0;
     PcgScalars h{};
+    int blocks;
+    const CgPlan plan = cg_plan(&R, 1, ctx->nsm, &blocks);
+    if (ctx->precond != SCDAT_PRECOND_MULTIGRID && plan.ok) {
+        ++ctx->launches;
+        CK(launch_cg_mixed(plan, A, ctx->b.p, ctx->x.p, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
+        int rc = read_group_scalars(ctx, h);
+        if (rc) return rc;
+        iters = h.iter;
+        relres = std::sqrt(h.rr / (h.bb > 0.0 ? h.bb : 1.0));
+        return SCDAT_OK;
+    }
     // every pass ends with the FP64 residual of the corrected x, so relres always describes the
     // returned solution, also when the pass cap ends the loop
     for (int outer = 0;; ++outer) {
@@ -930,10 +966,11 @@ int create_ctx(const scdat_mesh_desc* mesh, const scdat_params* params, scdat_ct
     pv.diagf = ctx->diagf.p;
     pv.dinvf = ctx->dinvf.p;
     size_t R = (size_t)std::max(ps.R, 1);
-    for (DBuf<double>* v : {&ctx->b, &ctx->x, &ctx->r, &ctx->z, &ctx->p, &ctx->pn, &ctx->q}) CK(v->alloc(R));
+    for (DBuf<double>* v : {&ctx->b, &ctx->x, &ctx->r, &ctx->z, &ctx->pn, &ctx->q}) CK(v->alloc(R));
     for (DBuf<float>* v : {&ctx->xf, &ctx->rf, &ctx->zf, &ctx->pf, &ctx->pnf, &ctx->qf}) CK(v->alloc(R));
+    CK(ctx->p.alloc(2 * R));  // the one-launch solve keeps z beside the direction
     CK(ctx->sc.alloc(1));
-    CK(ctx->part.alloc((size_t)ctx->grid_red * 4));
+    CK(ctx->part.alloc(std::max((size_t)ctx->grid_red * 4, kCgSlotBytes / sizeof(double))));
     // fields
     CK(ctx->rho.alloc((size_t)m.N));
     CK(ctx->tmp_rho.alloc((size_t)m.N));

@@ -5,7 +5,9 @@
 // field solve.
 #include "../../include/scdat_b200.h"
 #include "pcg_csr.cuh"
+#include "pcg_group.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -16,12 +18,13 @@ __global__ void k_reciprocal(int R, const double* __restrict__ d, double* __rest
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) out[i] = 1.0 / d[i];
 }
 
-// Device scratch of one solve: 6 R-vectors, the scalars and the reduction partials.
+// Device scratch of one solve: 6 R-vectors, the scalars and the reduction partials (or the
+// one-launch solve's barrier slots).
 size_t pcg_scratch_bytes(int R, int grid)
 {
     size_t v = (size_t)R * sizeof(double);
     v = (v + 255) & ~(size_t)255;
-    return 6 * v + 256 + (((size_t)grid * 4 * sizeof(double) + 255) & ~(size_t)255);
+    return 6 * v + 256 + std::max((((size_t)grid * 4 * sizeof(double) + 255) & ~(size_t)255), kCgSlotBytes);
 }
 
 PcgScratch pcg_scratch_carve(void* base, int R, int grid)
@@ -53,13 +56,27 @@ cudaError_t pcg_csr_run(int R, const int32_t* row_ptr, const int32_t* col, const
     A.col = col;
     A.val = val;
     A.diag = diag;
+    PcgScalars h{};
+    cudaError_t e;
+    int dev = 0, nsm = 0, blocks;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const CgPlan plan = cg_plan(&R, 1, nsm, &blocks);
+    if (plan.ok) {
+        // s.p and s.pn lie one behind the other: the 2 R values of the direction and z
+        if ((e = launch_cg64(plan, A, b, x, s.p, s.sc, s.part, rtol, max_iter, st)) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(&h, s.sc, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+        if (h.done < 0) return cudaErrorLaunchTimeout;
+        if (iters) *iters = h.iter;
+        if (relres) *relres = std::sqrt(h.rr / (h.bb > 0.0 ? h.bb : 1.0));
+        return cudaGetLastError();
+    }
     A.dinv = s.dinv;
     k_reciprocal<<<grid, 256, 0, st>>>(R, diag, s.dinv);
-    PcgScalars h{};
     h.rtol = rtol;
     h.max_iter = max_iter;
-    cudaError_t e = cudaMemcpyAsync(s.sc, &h, sizeof(h), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(s.sc, &h, sizeof(h), cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
     launch_pcg_init64(A, b, x, s.r, s.z, s.sc, s.part, grid, st);
     double* p = s.p;
     double* pn = s.pn;

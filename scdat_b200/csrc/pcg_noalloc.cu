@@ -9,6 +9,7 @@
 // keeps until the process exits.
 #include "../../include/scdat_b200.h"
 #include "pcg_csr.cuh"
+#include "pcg_group.cuh"
 
 #include <mutex>
 
@@ -17,7 +18,8 @@ namespace {
 constexpr int kNoAllocGrid = 148 * 4;
 constexpr int kNoAllocMaxRows = 1 << 18;  // 262,144 rows: about 12.6 MB of scratch
 constexpr size_t kVecBytes = (((size_t)kNoAllocMaxRows * sizeof(double)) + 255) & ~(size_t)255;
-constexpr size_t kScratchBytes = 6 * kVecBytes + 256 + ((((size_t)kNoAllocGrid * 4 * sizeof(double)) + 255) & ~(size_t)255);
+constexpr size_t kPartBytes = (((size_t)kNoAllocGrid * 4 * sizeof(double)) + 255) & ~(size_t)255;
+constexpr size_t kScratchBytes = 6 * kVecBytes + 256 + (kPartBytes > scdat::kCgSlotBytes ? kPartBytes : scdat::kCgSlotBytes);
 
 __device__ __align__(256) unsigned char g_pcg_scratch[kScratchBytes];
 
