@@ -86,8 +86,10 @@ struct BlockMap {
 // counter ctr[pass - 1].
 void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int grid, int64_t* chunk_prefix, unsigned* ctr,
                          cudaStream_t st);
+// collide: some job's collisions draw for every particle (draws_for_all).
+bool draws_for_all(const SpeciesDev& S, const PushParams& pp);
 void launch_push_mixed_batch(const PushJob* jobs, int njobs, const int64_t* chunk_prefix, unsigned* ctr, int pass,
-                             int grid, cudaStream_t st);
+                             bool collide, int grid, cudaStream_t st);
 void launch_batch_refresh_trec(const FieldJob* jobs, const BlockMap& tets, cudaStream_t st);
 
 // field (batch_field.cu).  cond_* are CUDA-graph conditional handles (0 outside a graph);

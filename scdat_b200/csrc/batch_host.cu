@@ -82,6 +82,7 @@ struct scdat_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     bool graph_ready = false;
+    bool collide = false;  // which pass 1 the jobs need (draws_for_all of any)
     int64_t steps = 0;
     double last_step_ms = 0.0;
 
@@ -123,6 +124,7 @@ int upload_jobs(scdat_batch* b)
 {
     std::vector<PushJob> pj;
     std::vector<FieldJob> fj;
+    bool collide = false;
     for (size_t j = 0; j < b->job_of.size(); ++j) {
         scdat_ctx* c = b->ctx[b->job_of[j].first];
         const int s = b->job_of[j].second;
@@ -136,9 +138,9 @@ int upload_jobs(scdat_batch* b)
         J.L = c->led.p;
         J.ke_acc = c->ke_acc.p;
         DeferBufs& d = *b->defer[j];
-        const unsigned cap = (unsigned)d.idx[0].n;
-        J.D1 = DeferList{b->dcount.p + 2 * j, cap, d.idx[0].p, d.it[0].p, d.rem[0].p, d.vs[0].p};
-        J.D2 = DeferList{b->dcount.p + 2 * j + 1, cap, d.idx[1].p, d.it[1].p, d.rem[1].p, d.vs[1].p};
+        J.D1 = DeferList{b->dcount.p + 2 * j, (unsigned)d.idx[0].n, d.idx[0].p, d.it[0].p, d.rem[0].p, d.vs[0].p};
+        J.D2 = DeferList{b->dcount.p + 2 * j + 1, (unsigned)d.idx[1].n, d.idx[1].p, d.it[1].p, d.rem[1].p, d.vs[1].p};
+        collide = collide || draws_for_all(J.S, J.pp);
         pj.push_back(J);
     }
     for (size_t k = 0; k < b->ctx.size(); ++k) {
@@ -192,6 +194,8 @@ int upload_jobs(scdat_batch* b)
         F.surf_n = (int64_t)c->surf_node.n;
         fj.push_back(F);
     }
+    if (collide != b->collide) b->release_graph();  // captured with the other pass 1
+    b->collide = collide;
     BCK(cudaMemcpyAsync(b->pjobs.p, pj.data(), sizeof(PushJob) * pj.size(), cudaMemcpyHostToDevice, b->st));
     BCK(cudaMemcpyAsync(b->fjobs.p, fj.data(), sizeof(FieldJob) * fj.size(), cudaMemcpyHostToDevice, b->st));
     return SCDAT_OK;
@@ -226,7 +230,7 @@ int enqueue_front(scdat_batch* b, cudaStream_t s)
     const int grid = b->nsm * b->tune.push_blocks_per_sm;
     for (int pass = 1; pass <= 3; ++pass) {
         launch_batch_prefix(b->pjobs.p, nj, pass, grid, b->prefix.p, b->pass_ctr.p, s);
-        launch_push_mixed_batch(b->pjobs.p, nj, b->prefix.p, b->pass_ctr.p, pass, grid, s);
+        launch_push_mixed_batch(b->pjobs.p, nj, b->prefix.p, b->pass_ctr.p, pass, b->collide, grid, s);
     }
     launch_batch_surface(b->fjobs.p, nc, s);
     launch_batch_finalize_rhs(b->fjobs.p, b->nodes.view, b->rows.view, s);
@@ -426,8 +430,9 @@ SCDAT_API int scdat_batch_create(int32_t n, scdat_ctx* const* ctxs, scdat_batch*
         for (int s = 0; s < (int)c->species.size(); ++s) {
             b->job_of.emplace_back(k, s);
             auto d = std::make_unique<DeferBufs>();
-            const size_t cap = (size_t)std::max<int64_t>(c->species[s].cap, 1) / 4 + 4096;
             for (int l = 0; l < 2; ++l) {
+                // pass 1 may defer a whole job; pass 2's overflow ends in pass 2
+                const size_t cap = (size_t)std::max<int64_t>(c->species[s].cap, 1) / (l ? 4 : 1) + 4096;
                 BCK(d->idx[l].alloc(cap));
                 BCK(d->it[l].alloc(cap));
                 BCK(d->rem[l].alloc(cap));

@@ -408,6 +408,16 @@ __device__ inline double sigma_elastic(const SpeciesDev& S, double e_ev)
     return s > 0.0 ? s : 0.0;
 }
 
+// False where mcc_elastic would return false after the null-collision selection draw alone (mode 2,
+// most particles); v2: the particle's squared speed.
+__device__ __forceinline__ bool mcc_candidate(const SpeciesDev& S, const PushParams& pp, uint32_t pid, double v2)
+{
+    if (S.mcc_mode != 2) return true;
+    const double vm = S.vmax ? (double)__uint_as_float(__ldg(S.vmax)) : 0.0;
+    if (!(vm > 0.0 && v2 <= vm * vm)) return true;
+    return !(select_uniform(pp.seed, pid, pp.step) >= S.mcc_n * S.mcc_sigma * vm * pp.dt + 1e-15);
+}
+
 // MonteCarloCollisionHandler::processCollisions for one elastic process
 // (CollisionAlgorithm.cpp:500-538, 189-210) with Philox streams (seed; id, step, 2|3).
 // mode 0: the reference's two draws against p = nu dt; mode 1: one draw against

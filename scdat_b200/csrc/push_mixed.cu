@@ -13,8 +13,9 @@
 // fx_red_word).
 //
 // Sub-steps run in passes so that warps stay converged: pass 1 gives every particle at most
-// kCap1 sub-steps and appends the unfinished ones to a list; pass 2 gives those up to kCap2
-// more; pass 3 finishes the rest.  The step structure is the reference's
+// kCap1 sub-steps and appends the unfinished ones to a list, with those whose end needs more than
+// the store (lost, perhaps colliding, to be located in FP64); pass 2 gives those up to kCap2 more
+// sub-steps; pass 3 finishes the rest.  The step structure is the reference's
 // CrossTetrahedron::integrateTrajectory (PICParticleAlgorithms.cpp:536-740).
 #include "batch.cuh"
 #include "push.cuh"
@@ -222,11 +223,65 @@ __device__ __forceinline__ void deposit_traj_f(const MeshView& M, const SpeciesD
     }
 }
 
+constexpr int kWalkQueue = 64;  // a warp's queue: up to 31 waiting and a chunk of 32 more
+// sub-step counts that mark a particle pass 1 deferred for the end of its step only
+constexpr int kItLost = -1;    // it left the mesh
+constexpr int kItFinish = -2;  // it may collide
+// ends of pass 1's sub-step besides kDone, kCapped and kLost
+enum { kFinish = 3, kRedo = 4 };  // end the step, or run the whole sub-step, in pass 2
+
 struct FlightF {
     float rx, ry, rz, vx, vy, vz;
     float rem, vstart;
     int cur, it;
 };
+
+// The gathered field of a sub-step at barycentrics l (zero outside the tet), its length in time, and
+// the velocity after its two half kicks; rec: the tet's record, whose first line is in L1 by then.
+__device__ __forceinline__ float kick_f(const float4* rec, const SpeciesDev& S, const PushParams& pp, const float l[4],
+                                        bool in, FlightF& f)
+{
+    const float qm = (float)S.qm;
+    float Ex = 0.f, Ey = 0.f, Ez = 0.f;
+    if (in) {  // E = E0 + sum_i lambda_i (E_i - E0), i = 1..3
+        const float4 c = __ldg(rec + 2), d = __ldg(rec + 3), e = __ldg(rec + 4), g = __ldg(rec + 5);
+        Ex = fmaf(l[1], d.x, fmaf(l[2], d.w, fmaf(l[3], e.z, c.y)));
+        Ey = fmaf(l[1], d.y, fmaf(l[2], e.x, fmaf(l[3], e.w, c.z)));
+        Ez = fmaf(l[1], d.z, fmaf(l[2], e.y, fmaf(l[3], g.x, c.w)));
+    }
+    float adt = f.rem;
+    const float Em = sqrtf(Ex * Ex + Ey * Ey + Ez * Ez);
+    if (Em > 1e-10f) {
+        const float acc = Em * fabsf(qm);
+        if (acc > 1e-10f && f.vstart > 1.0f) adt = fminf(adt, 0.1f * f.vstart / acc);
+    }
+    adt = fmaxf(adt, f.rem * (float)pp.floor_ratio);
+    adt = fminf(adt, f.rem);
+    if (fabsf(qm) > 1e-20f) {
+        const float h = 2.0f * (qm * (0.5f * adt));
+        f.vx = fmaf(h, Ex, f.vx);
+        f.vy = fmaf(h, Ey, f.vy);
+        f.vz = fmaf(h, Ez, f.vz);
+    }
+    return adt;
+}
+
+// Deposit of a sub-step that stayed in its tet, from barycentrics l to le along (tx, ty, tz): the
+// symmetric sample points sum to q w lambda(midpoint) for the segment-cloud and Gauss-3 kernels.
+__device__ __forceinline__ void deposit_in_f(const float4* rec, const SpeciesDev& S, const PushParams& pp,
+                                             const float l[4], const float le[4], float tx, float ty, float tz,
+                                             ChargeAcc A)
+{
+    const double qw = S.q * S.w;
+    const bool tiny = sqrtf(tx * tx + ty * ty + tz * tz) < 1e-15f;
+    const int4 nd4 = __ldg(reinterpret_cast<const int4*>(rec) + 6);
+    const int nd[4] = {nd4.x, nd4.y, nd4.z, nd4.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float lk = tiny ? l[q] : (pp.dep_kernel == 0 ? le[q] : 0.5f * (l[q] + le[q]));
+        fx_red_word(A, nd[q], (qw * (double)lk) * pp.inv_uq);
+    }
+}
 
 // Run sub-steps until the step's time is used up, the particle is lost, or `cap` sub-steps
 // ran in this call.
@@ -234,9 +289,6 @@ __device__ __forceinline__ int advance_f(const MeshView& M, const SpeciesDev& S,
                                          int cap, ChargeAcc A,
                                          unsigned& nsub)
 {
-    const float qm = (float)S.qm;
-    const float floor_ratio = (float)pp.floor_ratio;
-    const double qw = S.q * S.w;
     // only J^-1 stays in registers; E0, the E differences and the node ids are read from the
     // record (already in L1) where they are used
     const float4* rec = reinterpret_cast<const float4*>(M.trec + 64 * (int64_t)f.cur);
@@ -250,28 +302,8 @@ __device__ __forceinline__ int advance_f(const MeshView& M, const SpeciesDev& S,
         if (k == cap) return kCapped;
         ++k;
         ++f.it;
-        float Ex = 0.f, Ey = 0.f, Ez = 0.f;
-        if (in) {  // E = E0 + sum_i lambda_i (E_i - E0), i = 1..3
-            const float4 c = __ldg(rec + 2), d = __ldg(rec + 3), e = __ldg(rec + 4), g = __ldg(rec + 5);
-            Ex = fmaf(l[1], d.x, fmaf(l[2], d.w, fmaf(l[3], e.z, c.y)));
-            Ey = fmaf(l[1], d.y, fmaf(l[2], e.x, fmaf(l[3], e.w, c.z)));
-            Ez = fmaf(l[1], d.z, fmaf(l[2], e.y, fmaf(l[3], g.x, c.w)));
-        }
-        float adt = f.rem;
-        float Em = sqrtf(Ex * Ex + Ey * Ey + Ez * Ez);
-        if (Em > 1e-10f) {
-            float acc = Em * fabsf(qm);
-            if (acc > 1e-10f && f.vstart > 1.0f) adt = fminf(adt, 0.1f * f.vstart / acc);
-        }
-        adt = fmaxf(adt, f.rem * floor_ratio);
-        adt = fminf(adt, f.rem);
         float sx = f.rx, sy = f.ry, sz = f.rz;
-        if (fabsf(qm) > 1e-20f) {
-            float h = 2.0f * (qm * (0.5f * adt));
-            f.vx = fmaf(h, Ex, f.vx);
-            f.vy = fmaf(h, Ey, f.vy);
-            f.vz = fmaf(h, Ez, f.vz);
-        }
+        const float adt = kick_f(rec, S, pp, l, in, f);
         f.rx = fmaf(f.vx, adt, f.rx);
         f.ry = fmaf(f.vy, adt, f.ry);
         f.rz = fmaf(f.vz, adt, f.rz);
@@ -280,15 +312,7 @@ __device__ __forceinline__ int advance_f(const MeshView& M, const SpeciesDev& S,
         if (inside_f(le)) {
             if (pp.deposit) {
                 if (in) {
-                    float tx = f.rx - sx, ty = f.ry - sy, tz = f.rz - sz;
-                    bool tiny = sqrtf(tx * tx + ty * ty + tz * tz) < 1e-15f;
-                    const int4 nd4 = __ldg(reinterpret_cast<const int4*>(rec) + 6);
-                    const int nd[4] = {nd4.x, nd4.y, nd4.z, nd4.w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        float lk = tiny ? l[q] : (pp.dep_kernel == 0 ? le[q] : 0.5f * (l[q] + le[q]));
-                        fx_red_word(A, nd[q], (qw * (double)lk) * pp.inv_uq);
-                    }
+                    deposit_in_f(rec, S, pp, l, le, f.rx - sx, f.ry - sy, f.rz - sz, A);
                 } else {
                     deposit_traj_f(M, S, pp, f.cur, J, sx, sy, sz, f.rx, f.ry, f.rz, A);
                 }
@@ -315,8 +339,43 @@ __device__ __forceinline__ int advance_f(const MeshView& M, const SpeciesDev& S,
     return f.it >= kMaxSubsteps ? kLost : kDone;
 }
 
-// End of a particle's step: boundary events for a lost particle, the statistics, the fused
-// MCC, and the store.
+// The collision of a particle that mcc_candidate let through: the new velocity in v, true on a hit.
+static __device__ __noinline__ bool collide_f(const SpeciesDev& S, const PushParams& pp, uint32_t pid, float v[3])
+{
+    double vx = v[0], vy = v[1], vz = v[2];
+    if (!mcc_elastic(S, pp, pid, vx, vy, vz)) return false;
+    v[0] = (float)vx; v[1] = (float)vy; v[2] = (float)vz;
+    return true;
+}
+
+// End of a particle's step in tet `tet` (< 0: inactive): the statistics, the fused MCC (with
+// COLLIDE; its draws out of line, since few particles reach them), and the store.
+template <bool COLLIDE>
+__device__ __forceinline__ void finish_in_f(const ParticleStore& P, const SpeciesDev& S, const PushParams& pp,
+                                            int64_t i, FlightF& f, int tet, double ke, PushStats& c)
+{
+    c.ke += ke;
+    if (tet >= 0) {
+        const double dvx = f.vx, dvy = f.vy, dvz = f.vz;
+        const double v2 = dvx * dvx + dvy * dvy + dvz * dvz;
+        c.ev |= kEvActive;
+        if (S.mcc_mode == 2) c.v2 = fmaxf(c.v2, (float)v2);  // the null-collision speed bound
+        if (COLLIDE && pp.do_mcc && S.mcc_enabled) {
+            const uint32_t pid = P.id[i];
+            if (mcc_candidate(S, pp, pid, v2)) {
+                float v[3] = {f.vx, f.vy, f.vz};
+                if (collide_f(S, pp, pid, v)) {
+                    c.ev |= kEvHit;
+                    f.vx = v[0]; f.vy = v[1]; f.vz = v[2];
+                }
+            }
+        }
+    }
+    mix_store(P, i, f.rx, f.ry, f.rz, f.vx, f.vy, f.vz);
+    P.tet[i] = tet;
+}
+
+// The same after the boundary events of a lost particle.
 __device__ __forceinline__ void finish_f(const MeshView& M, const ParticleStore& P, const SpeciesDev& S,
                                          const PushParams& pp, LedgerDev* L, int64_t i, FlightF& f, int st,
                                          PushStats& c)
@@ -344,17 +403,7 @@ __device__ __forceinline__ void finish_f(const MeshView& M, const ParticleStore&
             f.rx = (float)px; f.ry = (float)py; f.rz = (float)pz;
         }
     }
-    c.ke += ke;
-    if (tet_out >= 0) {
-        c.ev |= kEvActive;
-        if (S.mcc_mode == 2) c.v2 = fmaxf(c.v2, (float)(dvx * dvx + dvy * dvy + dvz * dvz));  // the null-collision speed bound
-        if (pp.do_mcc && S.mcc_enabled && mcc_elastic(S, pp, P.id[i], dvx, dvy, dvz)) {
-            c.ev |= kEvHit;
-            f.vx = (float)dvx; f.vy = (float)dvy; f.vz = (float)dvz;
-        }
-    }
-    mix_store(P, i, f.rx, f.ry, f.rz, f.vx, f.vy, f.vz);
-    P.tet[i] = tet_out;
+    finish_in_f<true>(P, S, pp, i, f, tet_out, ke, c);
 }
 
 __device__ __forceinline__ void defer_store_f(const ParticleStore& P, const DeferList& D, unsigned slot, int64_t i,
@@ -387,15 +436,148 @@ __device__ __forceinline__ void load_first(const ParticleStore& P, const SortedS
     }
 }
 
-// Pass 1 for the 32 particles [base, base + 32) of one warp: at most kCap1 sub-steps, the
-// unfinished ones appended to D.
+// A warp's particles that left their tet in pass 1 and wait for their walk: the state after the
+// kick, with the drift still to be done (its end point is fmaf(v, adt, s), as the sub-step computed it).
+struct WalkQueue {
+    uint32_t i[kWalkQueue];
+    int cur[kWalkQueue];
+    float sx[kWalkQueue], sy[kWalkQueue], sz[kWalkQueue], vx[kWalkQueue], vy[kWalkQueue], vz[kWalkQueue];
+    float adt[kWalkQueue], vstart[kWalkQueue];
+};
+
+__device__ __forceinline__ WalkQueue& walk_queue()
+{
+    __shared__ WalkQueue q[8];
+    return q[threadIdx.x >> 5];
+}
+
+// End of a particle's pass-1 sub-step.  Finished particles are stored; the others go to D, where
+// whole warps of them are worked through: kCapped (time left), kLost and kFinish (entered with `it` =
+// kItLost, kItFinish), kRedo (f holds the state of the step's start).  Whatever is rare or needs a
+// call is one of those, so the pass-1 kernels carry no call and keep nothing in local memory (with
+// the calls inline 600 bytes of spills, a third of the launch's L1 sectors).  D holds the whole
+// species, so nothing overflows.  COLLIDE: collision modes that draw for every particle end here.
+template <bool COLLIDE>
+__device__ __forceinline__ void end_first(const ParticleStore& P, const SpeciesDev& S, const PushParams& pp,
+                                          const DeferList& D, LedgerDev* L, int64_t i, FlightF& f, int st,
+                                          PushStats& c)
+{
+    double ke = 0.0;
+    if (st == kDone) {
+        const double dvx = f.vx, dvy = f.vy, dvz = f.vz;
+        const double v2 = dvx * dvx + dvy * dvy + dvz * dvz;
+        ke = 0.5 * S.m * v2;
+        if (!COLLIDE && pp.do_mcc && S.mcc_enabled && mcc_candidate(S, pp, P.id[i], v2)) st = kFinish;
+    }
+    const bool more = st > kDone;
+    const unsigned slot = warp_append(more, D.count);
+    if (more) {
+        f.it = st == kLost ? kItLost : (st == kFinish ? kItFinish : f.it);
+        if (slot < D.cap) {
+            defer_store_f(P, D, slot, i, f);
+        } else {
+            // the step fails with this flag; the particle is stored as it stands
+            atomicOr(&L->flags, (unsigned long long)kFlagDeferOverflow);
+            mix_store(P, i, f.rx, f.ry, f.rz, f.vx, f.vy, f.vz);
+            P.tet[i] = f.cur;
+        }
+    } else if (st == kDone) {
+        finish_in_f<COLLIDE>(P, S, pp, i, f, f.cur, ke, c);
+    }
+    warp_chunk_end(c);
+}
+
+// Walks m (up to 32) particles of the warp's queue from position `first` on: relocate_f's walk and
+// the deposit in the tet it ends in, then end_first.
+template <bool COLLIDE>
+__device__ __forceinline__ void walk_queued(const MeshView& M, const ParticleStore& P, const SortedSource& R,
+                                            const SpeciesDev& S, const PushParams& pp, const DeferList& D, ChargeAcc A,
+                                            LedgerDev* L, int first, int m, PushStats& c)
+{
+    const int lane = threadIdx.x & 31;
+    const WalkQueue& Q = walk_queue();
+    const int e = first + lane;
+    int st = -1;
+    int64_t i = 0;
+    FlightF f;
+    __syncwarp();
+    if (lane < m) {
+        i = Q.i[e];
+        const int cur = Q.cur[e];
+        const float adt = Q.adt[e];
+        float sx = Q.sx[e], sy = Q.sy[e], sz = Q.sz[e];
+        float qx = fmaf(Q.vx[e], adt, sx), qy = fmaf(Q.vy[e], adt, sy), qz = fmaf(Q.vz[e], adt, sz);
+        int t = cur;
+        bool found = false;
+        float J[9];
+        {
+            float ox = 0.f, oy = 0.f, oz = 0.f, l[4];
+            load_j(M, t, J);
+            baryj(J, qx, qy, qz, l);
+            for (int k = 0; k < kWalkSteps; ++k) {
+                int fc = 0;
+                float lm = l[0];
+                if (l[1] < lm) { lm = l[1]; fc = 1; }
+                if (l[2] < lm) { lm = l[2]; fc = 2; }
+                if (l[3] < lm) fc = 3;
+                const float4 sh = __ldg(reinterpret_cast<const float4*>(M.trec + 64 * (int64_t)t) + 8 + fc);
+                const int nt = __float_as_int(sh.w);
+                if (nt < 0) break;
+                qx += sh.x; qy += sh.y; qz += sh.z;
+                ox += sh.x; oy += sh.y; oz += sh.z;
+                t = nt;
+                load_j(M, t, J);
+                baryj(J, qx, qy, qz, l);
+                found = inside_f(l);
+                if (found || !(l[0] == l[0])) break;
+            }
+            sx += ox; sy += oy; sz += oz;
+        }
+        f.vstart = Q.vstart[e];
+        if (found) {
+            if (pp.deposit) deposit_traj_f(M, S, pp, t, J, sx, sy, sz, qx, qy, qz, A);
+            ++c.nsub;
+            f.cur = t;
+            f.rx = qx; f.ry = qy; f.rz = qz;
+            f.vx = Q.vx[e]; f.vy = Q.vy[e]; f.vz = Q.vz[e];
+            f.rem = (float)pp.dt - adt;
+            f.it = 1;
+            st = f.rem > 1e-20f ? kCapped : kDone;
+        } else {
+            // a boundary face or a long walk: out of the domain, or (into the body, or in doubt) run
+            // again by pass 2, which locates in FP64
+            f.cur = cur;
+            f.vx = Q.vx[e]; f.vy = Q.vy[e]; f.vz = Q.vz[e];
+            f.rx = fmaf(f.vx, adt, Q.sx[e]); f.ry = fmaf(f.vy, adt, Q.sy[e]); f.rz = fmaf(f.vz, adt, Q.sz[e]);
+            const double3 o = origin(M, cur);
+            st = kLost;
+            if (!outside_grid(M, o.x + (double)f.rx, o.y + (double)f.ry, o.z + (double)f.rz)) {
+                load_first(P, R, i, f);
+                f.cur = cur;
+                f.rem = (float)pp.dt;
+                f.it = 0;
+                st = kRedo;
+            }
+        }
+    }
+    end_first<COLLIDE>(P, S, pp, D, L, i, f, st, c);
+}
+
+// Pass 1 for the 32 particles [base, base + 32) of one warp: one sub-step (kCap1).  It is run
+// here up to the test whether the particle is still in its tet; those that are not wait in the
+// warp's queue (`queued` so far) until 32 of them can walk together.
+template <bool COLLIDE>
 __device__ __forceinline__ void push1_warp(const MeshView& M, const ParticleStore& P, const SortedSource& R,
                                            const SpeciesDev& S, const PushParams& pp, const DeferList& D, ChargeAcc A,
-                                           LedgerDev* L, int64_t base, int64_t n, PushStats& c)
+                                           LedgerDev* L, int64_t base, int64_t n, int& queued, PushStats& c)
 {
-    const int64_t i = base + (threadIdx.x & 31);
+    static_assert(kCap1 == 1, "pass 1 runs one sub-step");
+    const int lane = threadIdx.x & 31;
+    const int64_t i = base + lane;
     int st = -1;
+    bool leaves = false;
     FlightF f;
+    float adt = 0.f;
     if (i < n) {
         load_first(P, R, i, f);
         if (f.cur <= kTetAbsorbed) {
@@ -406,30 +588,51 @@ __device__ __forceinline__ void push1_warp(const MeshView& M, const ParticleStor
             f.vstart = sqrtf(f.vx * f.vx + f.vy * f.vy + f.vz * f.vz);
             f.rem = (float)pp.dt;
             f.it = 0;
-            st = kDone;
-            if (f.cur < 0) {
-                // no hint: the stored offset is an absolute position
-                double px = f.rx, py = f.ry, pz = f.rz;
-                int t = locate_far(M, px, py, pz, -1);
-                if (t < 0) {
-                    st = kLost;
+            st = f.cur < 0 ? kRedo : kDone;  // no hint: located by pass 2
+            if (st == kDone && f.rem > 1e-20f) {
+                const float4* rec = reinterpret_cast<const float4*>(M.trec + 64 * (int64_t)f.cur);
+                float J[9], l[4], le[4];
+                load_j(M, f.cur, J);
+                baryj(J, f.rx, f.ry, f.rz, l);
+                const bool in = inside_f(l);
+                const float sx = f.rx, sy = f.ry, sz = f.rz;
+                adt = kick_f(rec, S, pp, l, in, f);
+                f.rx = fmaf(f.vx, adt, sx);
+                f.ry = fmaf(f.vy, adt, sy);
+                f.rz = fmaf(f.vz, adt, sz);
+                baryj(J, f.rx, f.ry, f.rz, le);
+                if (inside_f(le)) {
+                    if (pp.deposit) {
+                        if (in)
+                            deposit_in_f(rec, S, pp, l, le, f.rx - sx, f.ry - sy, f.rz - sz, A);
+                        else
+                            deposit_traj_f(M, S, pp, f.cur, J, sx, sy, sz, f.rx, f.ry, f.rz, A);
+                    }
+                    f.rem -= adt;
+                    f.it = 1;
+                    ++c.nsub;
+                    if (f.rem > 1e-20f) st = kCapped;
                 } else {
-                    double3 o = origin(M, t);
-                    f.rx = (float)(px - o.x); f.ry = (float)(py - o.y); f.rz = (float)(pz - o.z);
-                    f.cur = t;
+                    leaves = true;
+                    f.rx = sx; f.ry = sy; f.rz = sz;
                 }
             }
-            if (st != kLost) st = advance_f(M, S, pp, f, kCap1, A, c.nsub);
         }
     }
-    unsigned slot = warp_append(st == kCapped, D.count);
-    if (st == kCapped && slot < D.cap) {
-        defer_store_f(P, D, slot, i, f);
-    } else if (st >= 0) {
-        if (st == kCapped) st = advance_f(M, S, pp, f, 0x7fffffff, A, c.nsub);
-        finish_f(M, P, S, pp, L, i, f, st, c);
+    const unsigned m = __ballot_sync(0xffffffffu, leaves);
+    if (leaves) {
+        const int e = queued + __popc(m & ((1u << lane) - 1u));
+        WalkQueue& Q = walk_queue();
+        Q.i[e] = (uint32_t)i;
+        Q.cur[e] = f.cur;
+        Q.sx[e] = f.rx; Q.sy[e] = f.ry; Q.sz[e] = f.rz;
+        Q.vx[e] = f.vx; Q.vy[e] = f.vy; Q.vz[e] = f.vz;
+        Q.adt[e] = adt;
+        Q.vstart[e] = f.vstart;
+        st = -1;
     }
-    warp_chunk_end(c);
+    queued += __popc(m);
+    end_first<COLLIDE>(P, S, pp, D, L, i, f, st, c);
 }
 
 // Pass 1's one sub-step for a species that rarely leaves its tet, with no walk code: the
@@ -442,7 +645,6 @@ __device__ __forceinline__ int advance_stay_f(const MeshView& M, const SpeciesDe
                                               FlightF& f, ChargeAcc A, unsigned& nsub)
 {
     if (!(f.rem > 1e-20f && f.it < kMaxSubsteps)) return f.it >= kMaxSubsteps ? kLost : kDone;
-    const float qm = (float)S.qm;
     const float4* rec = reinterpret_cast<const float4*>(M.trec + 64 * (int64_t)f.cur);
     float l[4];
     {
@@ -451,25 +653,9 @@ __device__ __forceinline__ int advance_stay_f(const MeshView& M, const SpeciesDe
         baryj(J, f.rx, f.ry, f.rz, l);
     }
     if (!inside_f(l)) return kCapped;
-    const float4 c = __ldg(rec + 2), d = __ldg(rec + 3), e = __ldg(rec + 4), g = __ldg(rec + 5);
-    const float Ex = fmaf(l[1], d.x, fmaf(l[2], d.w, fmaf(l[3], e.z, c.y)));
-    const float Ey = fmaf(l[1], d.y, fmaf(l[2], e.x, fmaf(l[3], e.w, c.z)));
-    const float Ez = fmaf(l[1], d.z, fmaf(l[2], e.y, fmaf(l[3], g.x, c.w)));
-    float adt = f.rem;
-    const float Em = sqrtf(Ex * Ex + Ey * Ey + Ez * Ez);
-    if (Em > 1e-10f) {
-        const float acc = Em * fabsf(qm);
-        if (acc > 1e-10f && f.vstart > 1.0f) adt = fminf(adt, 0.1f * f.vstart / acc);
-    }
-    adt = fmaxf(adt, f.rem * (float)pp.floor_ratio);
-    adt = fminf(adt, f.rem);
-    float vx = f.vx, vy = f.vy, vz = f.vz;
-    if (fabsf(qm) > 1e-20f) {
-        const float h = 2.0f * (qm * (0.5f * adt));
-        vx = fmaf(h, Ex, vx);
-        vy = fmaf(h, Ey, vy);
-        vz = fmaf(h, Ez, vz);
-    }
+    FlightF g = f;
+    const float adt = kick_f(rec, S, pp, l, true, g);
+    const float vx = g.vx, vy = g.vy, vz = g.vz;
     const float rx = fmaf(vx, adt, f.rx), ry = fmaf(vy, adt, f.ry), rz = fmaf(vz, adt, f.rz);
     float le[4];
     {
@@ -479,18 +665,7 @@ __device__ __forceinline__ int advance_stay_f(const MeshView& M, const SpeciesDe
     }
     if (!inside_f(le)) return kCapped;
     ++f.it;
-    if (pp.deposit) {
-        const double qw = S.q * S.w;
-        const float tx = rx - f.rx, ty = ry - f.ry, tz = rz - f.rz;
-        const bool tiny = sqrtf(tx * tx + ty * ty + tz * tz) < 1e-15f;
-        const int4 nd4 = __ldg(reinterpret_cast<const int4*>(rec) + 6);
-        const int nd[4] = {nd4.x, nd4.y, nd4.z, nd4.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float lk = tiny ? l[q] : (pp.dep_kernel == 0 ? le[q] : 0.5f * (l[q] + le[q]));
-            fx_red_word(A, nd[q], (qw * (double)lk) * pp.inv_uq);
-        }
-    }
+    if (pp.deposit) deposit_in_f(rec, S, pp, l, le, rx - f.rx, ry - f.ry, rz - f.rz, A);
     f.rx = rx; f.ry = ry; f.rz = rz;
     f.vx = vx; f.vy = vy; f.vz = vz;
     f.rem -= adt;
@@ -501,6 +676,7 @@ __device__ __forceinline__ int advance_stay_f(const MeshView& M, const SpeciesDe
 // Stay-first pass 1 for the 32 particles [base, base + 32): one sub-step for those that stay in
 // their tet; everything else (leaving the tet, more time left, no location hint) goes to D,
 // whose capacity covers the whole species, so nothing overflows.
+template <bool COLLIDE>
 __device__ __forceinline__ void push1_stay_warp(const MeshView& M, const ParticleStore& P, const SortedSource& R,
                                                 const SpeciesDev& S, const PushParams& pp, const DeferList& D,
                                                 ChargeAcc A, LedgerDev* L, int64_t base, int64_t n, PushStats& c)
@@ -520,20 +696,7 @@ __device__ __forceinline__ void push1_stay_warp(const MeshView& M, const Particl
             st = f.cur < 0 ? kCapped : advance_stay_f(M, S, pp, f, A, c.nsub);
         }
     }
-    const unsigned slot = warp_append(st == kCapped, D.count);
-    if (st == kCapped) {
-        if (slot < D.cap) {
-            defer_store_f(P, D, slot, i, f);
-        } else {
-            // the step fails with this flag; the particle is stored as it stands
-            atomicOr(&L->flags, (unsigned long long)kFlagDeferOverflow);
-            mix_store(P, i, f.rx, f.ry, f.rz, f.vx, f.vy, f.vz);
-            P.tet[i] = f.cur;
-        }
-    } else if (st >= 0) {
-        finish_f(M, P, S, pp, L, i, f, st, c);
-    }
-    warp_chunk_end(c);
+    end_first<COLLIDE>(P, S, pp, D, L, i, f, st, c);
 }
 
 // Passes 2 and 3 for entries [base, base + 32) of list Din (up to `cap` sub-steps, then
@@ -555,9 +718,10 @@ __device__ __forceinline__ void push_more_warp(const MeshView& M, const Particle
         f.it = Din.it[e];
         f.rem = (float)Din.rem[e];
         f.vstart = (float)Din.vstart[e];
-        st = kDone;
-        if (f.cur < 0) {
-            // no location hint (only a stay-first pass 1 defers these): locate the absolute position
+        const bool ends = f.it < 0;  // kItLost, kItFinish: only the end of the step is left
+        st = f.it == kItLost ? kLost : kDone;
+        if (!ends && f.cur < 0) {
+            // no location hint: locate the absolute position
             const double px = f.rx, py = f.ry, pz = f.rz;
             const int t = locate_far(M, px, py, pz, -1);
             if (t < 0) {
@@ -568,7 +732,7 @@ __device__ __forceinline__ void push_more_warp(const MeshView& M, const Particle
                 f.cur = t;
             }
         }
-        if (st != kLost) st = advance_f(M, S, pp, f, chain ? cap : 0x7fffffff, A, c.nsub);
+        if (!ends && st != kLost) st = advance_f(M, S, pp, f, chain ? cap : 0x7fffffff, A, c.nsub);
     }
     unsigned slot = chain ? warp_append(st == kCapped, Dout.count) : 0xffffffffu;
     if (st == kCapped && chain && slot < Dout.cap) {
@@ -581,12 +745,16 @@ __device__ __forceinline__ void push_more_warp(const MeshView& M, const Particle
 }
 
 // Pass 1: every stored particle.  Warps take runs of 32-particle chunks from the launch's
-// work counter until none are left, so no warp idles while another still has work.
-// 5 blocks of 256 per SM (48 registers): with the record's vector loads and the folded re-sort
-// gather, the fewer spills now pay more than the sixth block's warps (push per step at 128^3:
-// 5 blocks 35.97 ms, 6 blocks 36.92, 4 blocks 40.2; the walk inlined: 36.11 at 6 blocks,
-// 37.56 at 5).
-__global__ void __launch_bounds__(256, 5) k_push_mixed(const __grid_constant__ MeshView M, ParticleStore P,
+// work counter until none are left, so no warp idles while another still has work.  What bounds it
+// is the latency of the records' dependent loads under divergence: with the walk, the boundary
+// events and the collisions in the chunk's own flow, 15 of 32 threads were active and the calls
+// cost 28 local-memory sectors a particle.  Walking from the warp's queue and ending the rare
+// cases in pass 2 took the electrons' launch at 64^3 cells, 64 ppc (16 M) from 2.30 to 1.41 ms,
+// with 21 of 32 threads active and no local memory.  4 blocks of 256 per SM (64 registers): 5
+// blocks spill 200 bytes (push per step at that size: 3 blocks 3.04 ms, 4 2.83, 5 3.06, 6 3.18).
+template <bool COLLIDE>
+__global__ void __launch_bounds__(256, 4) k_push_mixed(const __grid_constant__ MeshView M,
+                                                    const __grid_constant__ ParticleStore P,
                                                     const __grid_constant__ SortedSource R,
                                                     const __grid_constant__ SpeciesDev S,
                                                     const __grid_constant__ PushParams pp, DeferList D, ChargeAcc A,
@@ -596,20 +764,32 @@ __global__ void __launch_bounds__(256, 5) k_push_mixed(const __grid_constant__ M
     PushStats c{0.0, 0u, 0u};
     const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
     warp_stats_begin();
-    for (;;) {
-        const int64_t b0 = (int64_t)next_chunk(ctr) * run;
-        if (b0 >= n) break;
-        for (int64_t base = b0; base < b0 + run && base < n; base += 32)
-            push1_warp(M, P, R, S, pp, D, A, L, base, n, c);
+    int64_t base = 0, end = 0;
+    int queued = 0;
+    for (bool left = true;;) {
+        if (queued >= 32 || (!left && queued > 0)) {
+            const int m = min(queued, 32);
+            queued -= m;
+            walk_queued<COLLIDE>(M, P, R, S, pp, D, A, L, queued, m, c);
+        } else if (!left) {
+            break;
+        } else if (base < end) {
+            push1_warp<COLLIDE>(M, P, R, S, pp, D, A, L, base, n, queued, c);
+            base += 32;
+        } else {
+            base = (int64_t)next_chunk(ctr) * run;
+            end = min(base + run, n);
+            left = base < n;
+        }
     }
     warp_stats_flush(L, ke_acc, S.vmax);
 }
 
-// Stay-first pass 1 (same work distribution as k_push_mixed); no walk code, so at 4 blocks of
-// 256 per SM it fits in 62 registers without spilling.  Its launch is bound by L1 wavefronts
-// (scattered record loads, one atomic per lane and node), so the spills of a denser launch cost
-// more than its extra warps gain: 4 blocks 37.66 ms of push per step at 128^3, 5 blocks
-// 38.5, 6 blocks (40 registers, 200 bytes of spill stores) 38.83.
+// Stay-first pass 1 (same work distribution as k_push_mixed), no walk code.  Its launch is bound by
+// L1 wavefronts (scattered record loads, one atomic per lane and node), so more warps gain nothing:
+// 16 M ions at 64^3 cells 4 blocks of 256 per SM 754 us, 5 blocks 748, 6 blocks 757, none of them
+// with spills.
+template <bool COLLIDE>
 __global__ void __launch_bounds__(256, 4) k_push_mixed_stay(const __grid_constant__ MeshView M, ParticleStore P,
                                                          const __grid_constant__ SortedSource R,
                                                          const __grid_constant__ SpeciesDev S,
@@ -625,13 +805,13 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_stay(const __grid_constan
         const int64_t b0 = (int64_t)next_chunk(ctr) * run;
         if (b0 >= n) break;
         for (int64_t base = b0; base < b0 + run && base < n; base += 32)
-            push1_stay_warp(M, P, R, S, pp, D, A, L, base, n, c);
+            push1_stay_warp<COLLIDE>(M, P, R, S, pp, D, A, L, base, n, c);
     }
     warp_stats_flush(L, ke_acc, S.vmax);
 }
 
-// Passes 2 and 3, 4 blocks of 256 per SM (64 registers; push per step at 128^3: 4 blocks 36.32
-// ms, 3 blocks 36.46, 5 blocks 36.55).
+// Passes 2 and 3, 4 blocks of 256 per SM (64 registers; the four launches of a step at 64^3 cells,
+// 64 ppc: 4 blocks 598 us, 3 blocks 610, 5 blocks 641).
 __global__ void __launch_bounds__(256, 4) k_push_mixed_more(const __grid_constant__ MeshView M, ParticleStore P,
                                                          const __grid_constant__ SpeciesDev S,
                                                          const __grid_constant__ PushParams pp, DeferList Din,
@@ -684,10 +864,67 @@ __global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int 
     }
 }
 
-// Pass `pass` (1, 2 or 3) of every job.  Warps take units g of the global index from the pass's
-// work counter (pass 1: runs of pre[njobs + 1] 32-particle chunks; passes 2 and 3: single chunks); unit g
-// belongs to the job j with pre[j] <= g < pre[j + 1], and a warp flushes its statistics into a
-// job's ledger when it moves on to another job.
+// job of unit g: pre[j] <= g < pre[j + 1]
+__device__ __forceinline__ int job_of_unit(const int64_t* pre, int njobs, int64_t g)
+{
+    int lo = 0, hi = njobs;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid] <= g)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Pass 1 of every job.  Warps take units g of the global index from the pass's work counter (runs
+// of pre[njobs + 1] 32-particle chunks); unit g belongs to the job j with pre[j] <= g < pre[j + 1],
+// and a warp finishes its queued walks and flushes its statistics into a job's ledger when it moves
+// on to another job.
+template <bool COLLIDE>
+__global__ void __launch_bounds__(256, 4) k_push_mixed_batch_first(const PushJob* __restrict__ jobs, int njobs,
+                                                                const int64_t* __restrict__ pre,
+                                                                unsigned* __restrict__ ctr)
+{
+    __shared__ int64_t spre[kMaxBatchJobs + 1];
+    for (int j = threadIdx.x; j <= njobs; j += blockDim.x) spre[j] = pre[j];
+    __syncthreads();
+    const int64_t total = spre[njobs], run = 32 * pre[njobs + 1];
+    PushStats c{0.0, 0u, 0u};
+    warp_stats_begin();
+    int64_t base = 0, end = 0, next_base = 0;
+    int cur = -1, next = -1, queued = 0;  // next >= 0: the unit at next_base of that job is taken
+    for (bool left = true;;) {
+        if (queued >= 32 || (queued > 0 && (!left || (next >= 0 && next != cur)))) {
+            const PushJob& J = jobs[cur];
+            const int m = min(queued, 32);
+            queued -= m;
+            walk_queued<COLLIDE>(J.M, J.P, SortedSource{}, J.S, J.pp, J.D1, J.A, J.L, queued, m, c);
+        } else if (base < end) {
+            const PushJob& J = jobs[cur];
+            push1_warp<COLLIDE>(J.M, J.P, SortedSource{}, J.S, J.pp, J.D1, J.A, J.L, base, end, queued, c);
+            base += 32;
+        } else if (!left || (next >= 0 && next != cur)) {
+            if (cur >= 0) warp_stats_flush(jobs[cur].L, jobs[cur].ke_acc, jobs[cur].S.vmax);
+            if (!left) break;
+            cur = next;
+        } else if (next >= 0) {
+            base = next_base;
+            end = min(base + run, *jobs[cur].P.count);
+            next = -1;
+        } else {
+            const int64_t g = (int64_t)next_chunk(ctr);
+            left = g < total;
+            if (left) {
+                next = job_of_unit(spre, njobs, g);
+                next_base = (g - spre[next]) * run;
+            }
+        }
+    }
+}
+
+// Pass 2 or 3 of every job: units are single chunks of the jobs' defer lists.
 template <int PASS>
 __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __restrict__ jobs, int njobs,
                                                           const int64_t* __restrict__ pre, unsigned* __restrict__ ctr)
@@ -696,32 +933,18 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __re
     for (int j = threadIdx.x; j <= njobs; j += blockDim.x) spre[j] = pre[j];
     __syncthreads();
     const int64_t total = spre[njobs];
-    const int64_t run = PASS == 1 ? 32 * pre[njobs + 1] : 32;
     PushStats c{0.0, 0u, 0u};
     warp_stats_begin();
     int cur = -1;
     for (;;) {
         const int64_t g = (int64_t)next_chunk(ctr + PASS - 1);
         if (g >= total) break;
-        int lo = 0, hi = njobs;  // spre[lo] <= g < spre[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (spre[mid] <= g)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        if (lo != cur) {
+        const int j = job_of_unit(spre, njobs, g);
+        if (j != cur) {
             if (cur >= 0) warp_stats_flush(jobs[cur].L, jobs[cur].ke_acc, jobs[cur].S.vmax);
-            cur = lo;
+            cur = j;
         }
         const PushJob& J = jobs[cur];
-        if (PASS == 1) {
-            const int64_t n = *J.P.count, b0 = (g - spre[cur]) * run;
-            for (int64_t base = b0; base < b0 + run && base < n; base += 32)
-                push1_warp(J.M, J.P, SortedSource{}, J.S, J.pp, J.D1, J.A, J.L, base, n, c);
-            continue;
-        }
         const int64_t base = (g - spre[cur]) * 32;
         if (PASS == 2) {
             const int64_t n = min((int64_t)*J.D1.count, (int64_t)J.D1.cap);
@@ -802,14 +1025,18 @@ __global__ void k_refresh_trec(int64_t T, const int4* __restrict__ tet, const do
         refresh_trec_part(g >> 2, (int)(g & 3), tet, E, trec);
 }
 
+// The collision mode draws Philox numbers for every particle (modes 0 and 1), so pass 1 ends them
+// itself; the null collision's few candidates go to pass 2.
+bool draws_for_all(const SpeciesDev& S, const PushParams& pp) { return pp.do_mcc && S.mcc_enabled && S.mcc_mode != 2; }
+
 void launch_push_mixed(const MeshView& M, const ParticleStore& P, const SortedSource& R, const SpeciesDev& S,
                        const PushParams& pp, const DeferList& D1, const DeferList& D2, ChargeAcc A, LedgerDev* L,
                        unsigned long long* ke_acc, unsigned* ctr, int grid, bool stay_first, cudaStream_t st)
 {
-    if (stay_first)
-        k_push_mixed_stay<<<grid, 256, 0, st>>>(M, P, R, S, pp, D1, A, L, ke_acc, ctr);
-    else
-        k_push_mixed<<<grid, 256, 0, st>>>(M, P, R, S, pp, D1, A, L, ke_acc, ctr);
+    const bool collide = draws_for_all(S, pp);
+    auto first = stay_first ? (collide ? k_push_mixed_stay<true> : k_push_mixed_stay<false>)
+                            : (collide ? k_push_mixed<true> : k_push_mixed<false>);
+    first<<<grid, 256, 0, st>>>(M, P, R, S, pp, D1, A, L, ke_acc, ctr);
     k_push_mixed_more<<<grid, 256, 0, st>>>(M, P, S, pp, D1, D2, kCap2, A, L, ke_acc, ctr + 1);
     DeferList none{};
     k_push_mixed_more<<<grid, 256, 0, st>>>(M, P, S, pp, D2, none, 0, A, L, ke_acc, ctr + 2);
@@ -840,10 +1067,12 @@ void launch_batch_prefix(const PushJob* jobs, int njobs, int pass, int grid, int
 }
 
 void launch_push_mixed_batch(const PushJob* jobs, int njobs, const int64_t* chunk_prefix, unsigned* ctr, int pass,
-                             int grid, cudaStream_t st)
+                             bool collide, int grid, cudaStream_t st)
 {
-    if (pass == 1)
-        k_push_mixed_batch<1><<<grid, 256, 0, st>>>(jobs, njobs, chunk_prefix, ctr);
+    if (pass == 1 && collide)
+        k_push_mixed_batch_first<true><<<grid, 256, 0, st>>>(jobs, njobs, chunk_prefix, ctr);
+    else if (pass == 1)
+        k_push_mixed_batch_first<false><<<grid, 256, 0, st>>>(jobs, njobs, chunk_prefix, ctr);
     else if (pass == 2)
         k_push_mixed_batch<2><<<grid, 256, 0, st>>>(jobs, njobs, chunk_prefix, ctr);
     else
