@@ -66,23 +66,26 @@ struct GatherArrays {
 };
 
 
-// Node charge accumulators of the FP64 form: each 128-bit contribution is split into 32-bit
-// limbs that go into three 64-bit words with return-free atomic adds (no thread waits on an
-// atomic), and the limbs are recombined exactly when the charge is read.  2^32 contributions
-// per node and step fit before a limb could wrap.  The precision form uses l0 alone, as one
+// Node charge accumulators of the FP64 form: the magnitude of each 128-bit contribution is split
+// into 32-bit limbs that are added to or subtracted from three 64-bit words with return-free
+// atomics (no thread waits on an atomic), and the limbs are recombined exactly when the charge is
+// read.  A contribution is less than the unit, so its high limb is zero and two atomics carry it,
+// whatever its sign.  2^31 contributions per node and step fit before a limb could wrap.  The precision form uses l0 alone, as one
 // word per node (fx_red_word), with l1 = h = nullptr.
 struct ChargeAcc {
-    unsigned long long* l0;  // bits 0..31 of each contribution
-    unsigned long long* l1;  // bits 32..63
-    unsigned long long* h;   // the signed high word
+    unsigned long long* l0;  // bits 0..31 of each contribution, signed
+    unsigned long long* l1;  // bits 32..63, signed
+    unsigned long long* h;   // the high word, signed
 };
 
-__device__ __forceinline__ void fx_red(const ChargeAcc& A, int node, const Fx128& v)
+__device__ __forceinline__ void fx_red(const ChargeAcc& A, int node, double v)
 {
-    unsigned long long a = v.lo & 0xffffffffull, b = v.lo >> 32;
-    if (a) atomicAdd(A.l0 + node, a);
-    if (b) atomicAdd(A.l1 + node, b);
-    if (v.hi) atomicAdd(A.h + node, (unsigned long long)v.hi);
+    const Fx128 m = fx_from_double(fabs(v));
+    const unsigned long long s = v < 0.0 ? ~0ull : 0ull;  // two's complement: (x ^ s) - s negates
+    const unsigned long long a = m.lo & 0xffffffffull, b = m.lo >> 32, h = (unsigned long long)m.hi;
+    if (a) atomicAdd(A.l0 + node, (a ^ s) - s);
+    if (b) atomicAdd(A.l1 + node, (b ^ s) - s);
+    if (h) atomicAdd(A.h + node, (h ^ s) - s);
 }
 
 // The precision form's accumulators: one signed 64-bit word per node in units of 2^-36 of
@@ -110,8 +113,8 @@ __host__ __device__ inline Fx128 fx_from_acc(const unsigned long long* l0, const
 
 __host__ __device__ inline Fx128 fx_from_limbs(unsigned long long l0, unsigned long long l1, unsigned long long h)
 {
-    Fx128 r{l0, (long long)h};
-    Fx128 m{l1 << 32, (long long)(l1 >> 32)};
+    Fx128 r{l0, (long long)h + ((long long)l0 >> 63)};
+    Fx128 m{l1 << 32, (long long)l1 >> 32};
     fx_add(r, m);
     return r;
 }

@@ -498,6 +498,12 @@ struct DeferList {
 };
 
 enum { kDone = 0, kCapped = 1, kLost = 2 };
+constexpr int kWalkQueue = 64;  // a warp's queue: up to 31 waiting and a chunk of 32 more
+// sub-step counts that mark a particle pass 1 deferred for the end of its step only
+constexpr int kItLost = -1;    // it left the mesh
+constexpr int kItFinish = -2;  // it may collide
+// ends of pass 1's sub-step besides kDone, kCapped and kLost
+enum { kFinish = 3, kRedo = 4 };  // end the step, or run the whole sub-step, in pass 2
 
 // Per-lane push statistics of the current 32-particle chunk (one particle per lane): its
 // kinetic energy, its sub-steps and its events (kEvLost | kEvActive | kEvHit).

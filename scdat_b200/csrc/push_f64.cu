@@ -4,55 +4,64 @@
 // per-sub-step trajectory deposit (:371-433), then the runtime boundary events
 // (PICCycle.cpp:1221-1379) and, when enabled, the elastic background MCC.
 //
-// Charge goes into per-species 128-bit fixed-point node accumulators staged per warp in
-// shared memory, so the deposit is exact and independent of thread order.  The nodal E of
-// each tet's 4 nodes is kept per tet (refreshed after every field solve), so the gather is
-// one load beside the tet's geometry.  Sub-steps run in passes (see push_mixed.cu) to keep
-// warps converged.
+// Charge goes into per-species 128-bit fixed-point node accumulators, so the deposit is exact and
+// independent of thread order.  The nodal E of each tet's 4 nodes is kept per tet (refreshed after
+// every field solve), so the gather is one load beside the tet's geometry.  Sub-steps run in passes
+// to keep warps converged, and pass 1 walks from a queue and ends the rare cases in pass 2, as in
+// push_mixed.cu.
 #include "push.cuh"
 
 namespace scdat {
 
-struct DepositAcc {
-    Fx128 n[4];
-    bool any;
+constexpr int kPushWarpsD = 8, kPushBlocksD = 2;  // pass 1: warps of a block, blocks per SM
+
+// The inverse Jacobian (row-major) and origin of a tet's record.
+struct TetGeom {
+    double j[9], o[3];
 };
 
-__device__ __forceinline__ void dep_point(DepositAcc& acc, const double lam[4], double cw, double inv_uq)
+__device__ __forceinline__ TetGeom load_geom(const MeshView& M, int t)
 {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        Fx128 f = fx_from_double((cw * lam[i]) * inv_uq);
-        fx_add(acc.n[i], f);
-    }
-    acc.any = true;
+    const double2* g2 = reinterpret_cast<const double2*>(M.geom + 16 * (int64_t)t);
+    const double2 a = __ldg(g2), b = __ldg(g2 + 1), c = __ldg(g2 + 2), d = __ldg(g2 + 3), e = __ldg(g2 + 4),
+                  f = __ldg(g2 + 5);
+    return TetGeom{{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x}, {e.y, f.x, f.y}};
 }
 
-// ChargeDepositor::depositChargeAlongTrajectory into the post-move tet t
-// (PICParticleAlgorithms.cpp:371-433); each sample point counts only when it lies in t.
-static __device__ __noinline__ void deposit_traj(const MeshView& M, const SpeciesDev& S, const PushParams& pp, int t,
-                                                 double sx, double sy, double sz, double ex, double ey, double ez,
-                                                 ChargeAcc A)
+// bary64 from a record already in registers
+__device__ __forceinline__ bool baryg(const TetGeom& g, double px, double py, double pz, double lam[4])
 {
-    DepositAcc acc;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc.n[i] = Fx128{0ull, 0ll};
-    acc.any = false;
-    double tx = ex - sx, ty = ey - sy, tz = ez - sz;
-    double lam[4];
+    const double dx = px - g.o[0], dy = py - g.o[1], dz = pz - g.o[2];
+    lam[1] = g.j[0] * dx + g.j[1] * dy + g.j[2] * dz;
+    lam[2] = g.j[3] * dx + g.j[4] * dy + g.j[5] * dz;
+    lam[3] = g.j[6] * dx + g.j[7] * dy + g.j[8] * dz;
+    lam[0] = 1.0 - lam[1] - lam[2] - lam[3];
+    return bary_inside(lam);
+}
+
+// ChargeDepositor::depositChargeAlongTrajectory into the post-move tet t, whose record is g
+// (PICParticleAlgorithms.cpp:371-433); each sample point counts only when it lies in t.
+__device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev& S, const PushParams& pp, int t,
+                                             const TetGeom& g, double sx, double sy, double sz, double ex, double ey,
+                                             double ez, ChargeAcc A)
+{
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    bool any = false;
+    const double tx = ex - sx, ty = ey - sy, tz = ez - sz;
     const double qw = S.q * S.w;
-    if (sqrt(tx * tx + ty * ty + tz * tz) < 1e-15) {
-        if (bary64(M, t, sx, sy, sz, lam)) dep_point(acc, lam, qw, pp.inv_uq);
-    } else if (pp.dep_kernel == 0) {  // NearestPoint
-        if (bary64(M, t, ex, ey, ez, lam)) dep_point(acc, lam, qw, pp.inv_uq);
+    const bool tiny = sqrt(tx * tx + ty * ty + tz * tz) < 1e-15;
+    if (tiny || pp.dep_kernel == 0) {  // a point: the start of a tiny move, NearestPoint's end
+        double lam[4];
+        any = tiny ? baryg(g, sx, sy, sz, lam) : baryg(g, ex, ey, ez, lam);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[i] = qw * lam[i];
     } else {
         // barycentrics are affine along the segment: lam(s + tau*tr) = lam_s + tau*dlam
-        const double* g = M.geom + 16 * (int64_t)t;
         double ls[4], dl[4];
-        bary64(M, t, sx, sy, sz, ls);
-        dl[1] = __ldg(g + 0) * tx + __ldg(g + 1) * ty + __ldg(g + 2) * tz;
-        dl[2] = __ldg(g + 3) * tx + __ldg(g + 4) * ty + __ldg(g + 5) * tz;
-        dl[3] = __ldg(g + 6) * tx + __ldg(g + 7) * ty + __ldg(g + 8) * tz;
+        baryg(g, sx, sy, sz, ls);
+        dl[1] = g.j[0] * tx + g.j[1] * ty + g.j[2] * tz;
+        dl[2] = g.j[3] * tx + g.j[4] * ty + g.j[5] * tz;
+        dl[3] = g.j[6] * tx + g.j[7] * ty + g.j[8] * tz;
         dl[0] = -dl[1] - dl[2] - dl[3];
         const int nseg = pp.nseg;
         if (pp.dep_kernel == 2) {  // QuadratureGauss3
@@ -64,23 +73,54 @@ static __device__ __noinline__ void deposit_traj(const MeshView& M, const Specie
                 for (int q = 0; q < 3; ++q) {
                     double tau = tc + th * gn[q];
                     double l[4] = {ls[0] + tau * dl[0], ls[1] + tau * dl[1], ls[2] + tau * dl[2], ls[3] + tau * dl[3]};
-                    if (bary_inside(l)) dep_point(acc, l, (S.q * gw[q] / (double)nseg) * S.w, pp.inv_uq);
+                    if (bary_inside(l)) {
+                        const double cw = (S.q * gw[q] / (double)nseg) * S.w;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) sum[i] += cw * l[i];
+                        any = true;
+                    }
                 }
             }
-        } else {  // LinearSegmentCloud
-            for (int sg = 0; sg < nseg; ++sg) {
-                double tau = ((double)sg + 0.5) / (double)nseg;
-                double l[4] = {ls[0] + tau * dl[0], ls[1] + tau * dl[1], ls[2] + tau * dl[2], ls[3] + tau * dl[3]};
-                if (bary_inside(l)) dep_point(acc, l, S.cw_seg, pp.inv_uq);
+        } else {
+            // LinearSegmentCloud: the points tau_k = (k + 1/2) / nseg inside the tet are those of one
+            // interval of k, whose sum is in closed form.  Its ends come from the faces' crossings
+            // and are settled by the containment test of the points next to them, so that they are
+            // the points a loop over all of them would take.
+            const auto in = [&](int k) {
+                const double tau = ((double)k + 0.5) / (double)nseg;
+                const double l[4] = {ls[0] + tau * dl[0], ls[1] + tau * dl[1], ls[2] + tau * dl[2], ls[3] + tau * dl[3]};
+                return bary_inside(l);
+            };
+            double lo = 0.0, hi = 1.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (dl[i] == 0.0) continue;  // the point tests decide
+                const double inv = 1.0 / dl[i];
+                const double a = (-kBaryEps - ls[i]) * inv, b = (1.0 + kBaryEps - ls[i]) * inv;
+                lo = fmax(lo, fmin(a, b));
+                hi = fmin(hi, fmax(a, b));
+            }
+            int ka = max(0, (int)fmin(ceil(lo * (double)nseg - 0.5), (double)nseg));
+            int kb = min(nseg - 1, (int)fmax(floor(hi * (double)nseg - 0.5), -1.0));
+            if (ka > 0 && in(ka - 1)) --ka;
+            if (kb < nseg - 1 && in(kb + 1)) ++kb;
+            while (ka <= kb && !in(ka)) ++ka;
+            while (kb >= ka && !in(kb)) --kb;
+            if (ka <= kb) {
+                const double n = (double)(kb - ka + 1);
+                const double st = 0.5 * n * (double)(ka + kb + 1) / (double)nseg;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[i] = S.cw_seg * (n * ls[i] + st * dl[i]);
+                any = true;
             }
         }
     }
-    if (!acc.any) return;
-    int4 tn = rec_nodes(M, t);
-    fx_red(A, tn.x, acc.n[0]);
-    fx_red(A, tn.y, acc.n[1]);
-    fx_red(A, tn.z, acc.n[2]);
-    fx_red(A, tn.w, acc.n[3]);
+    if (!any) return;
+    const int4 tn = rec_nodes(M, t);
+    fx_red(A, tn.x, sum[0] * pp.inv_uq);
+    fx_red(A, tn.y, sum[1] * pp.inv_uq);
+    fx_red(A, tn.z, sum[2] * pp.inv_uq);
+    fx_red(A, tn.w, sum[3] * pp.inv_uq);
 }
 
 struct FlightD {
@@ -89,82 +129,115 @@ struct FlightD {
     int cur, it;
 };
 
+// The gathered field of a sub-step at barycentrics lam (zero outside the tet), its length in time
+// (CrossTetrahedron::adaptiveTimeStep with |B| = 0), and the velocity after its two half kicks.
+__device__ __forceinline__ double kick_d(const MeshView& M, const SpeciesDev& S, const PushParams& pp,
+                                         const double lam[4], bool in, FlightD& f)
+{
+    const double qm = S.qm;
+    double Ex = 0.0, Ey = 0.0, Ez = 0.0;
+    if (in) {
+        const double2* e2 = reinterpret_cast<const double2*>(M.erec + 12 * (int64_t)f.cur);
+        const double2 a = __ldg(e2), b = __ldg(e2 + 1), c = __ldg(e2 + 2), d = __ldg(e2 + 3), g = __ldg(e2 + 4),
+                      h = __ldg(e2 + 5);
+        const double e[12] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, g.x, g.y, h.x, h.y};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            Ex = Ex + e[3 * q] * lam[q];
+            Ey = Ey + e[3 * q + 1] * lam[q];
+            Ez = Ez + e[3 * q + 2] * lam[q];
+        }
+    }
+    double adt = f.rem;
+    const double Em = sqrt(Ex * Ex + Ey * Ey + Ez * Ez);
+    if (Em > 1e-10) {
+        const double acc = Em * fabs(qm);
+        if (acc > 1e-10 && f.vstart > 1.0) adt = fmin(adt, 0.1 * f.vstart / acc);
+    }
+    adt = fmax(adt, f.rem * pp.floor_ratio);
+    adt = fmin(adt, f.rem);
+    if (fabs(qm) > 1e-20) {
+        const double h = qm * (0.5 * adt);
+        f.vx = f.vx + Ex * h; f.vy = f.vy + Ey * h; f.vz = f.vz + Ez * h;
+        f.vx = f.vx + Ex * h; f.vy = f.vy + Ey * h; f.vz = f.vz + Ez * h;
+    }
+    return adt;
+}
+
+// Deposit of a sub-step that stayed in its tet (see deposit_in_f in push_mixed.cu).
+__device__ __forceinline__ void deposit_in_d(const MeshView& M, const SpeciesDev& S, const PushParams& pp, int t,
+                                             const double lam[4], const double le[4], double tx, double ty, double tz,
+                                             ChargeAcc A)
+{
+    const double qw = S.q * S.w;
+    const bool tiny = sqrt(tx * tx + ty * ty + tz * tz) < 1e-15;
+    const int4 tn = rec_nodes(M, t);
+    const int nd[4] = {tn.x, tn.y, tn.z, tn.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double lk = tiny ? lam[q] : (pp.dep_kernel == 0 ? le[q] : 0.5 * (lam[q] + le[q]));
+        fx_red(A, nd[q], (qw * lk) * pp.inv_uq);
+    }
+}
+
 // Run sub-steps until the step's time is used up, the particle is lost, or `cap` sub-steps
 // ran in this call.
 __device__ __forceinline__ int advance_d(const MeshView& M, const SpeciesDev& S, const PushParams& pp, FlightD& f,
                                          int cap, ChargeAcc A,
                                          unsigned& nsub)
 {
-    const double qm = S.qm;
-    const double qw = S.q * S.w;
+    TetGeom g = load_geom(M, f.cur);
     double lam[4];
-    bool in = bary64(M, f.cur, f.px, f.py, f.pz, lam);  // reused as the next gather's weights
+    bool in = baryg(g, f.px, f.py, f.pz, lam);  // reused as the next gather's weights
     int k = 0;
     while (f.rem > kMinTimeStep && f.it < kMaxSubsteps) {
         if (k == cap) return kCapped;
         ++k;
         ++f.it;
-        double Ex = 0.0, Ey = 0.0, Ez = 0.0;
-        if (in) {
-            const double* e = M.erec + 12 * (int64_t)f.cur;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                Ex = Ex + __ldg(e + 3 * q) * lam[q];
-                Ey = Ey + __ldg(e + 3 * q + 1) * lam[q];
-                Ez = Ez + __ldg(e + 3 * q + 2) * lam[q];
-            }
-        }
-        // CrossTetrahedron::adaptiveTimeStep with |B| = 0
-        double adt = f.rem;
-        double Em = sqrt(Ex * Ex + Ey * Ey + Ez * Ez);
-        if (Em > 1e-10) {
-            double acc = Em * fabs(qm);
-            if (acc > 1e-10 && f.vstart > 1.0) adt = fmin(adt, 0.1 * f.vstart / acc);
-        }
-        adt = fmax(adt, f.rem * pp.floor_ratio);
-        adt = fmin(adt, f.rem);
         const double sx = f.px, sy = f.py, sz = f.pz;
-        if (fabs(qm) > 1e-20) {
-            double h = qm * (0.5 * adt);
-            f.vx = f.vx + Ex * h; f.vy = f.vy + Ey * h; f.vz = f.vz + Ez * h;
-            f.vx = f.vx + Ex * h; f.vy = f.vy + Ey * h; f.vz = f.vz + Ez * h;
-        }
-        f.px = f.px + f.vx * adt;
-        f.py = f.py + f.vy * adt;
-        f.pz = f.pz + f.vz * adt;
+        const double adt = kick_d(M, S, pp, lam, in, f);
+        f.px = fma(f.vx, adt, sx);
+        f.py = fma(f.vy, adt, sy);
+        f.pz = fma(f.vz, adt, sz);
         double le[4];
-        if (bary64(M, f.cur, f.px, f.py, f.pz, le)) {
+        if (baryg(g, f.px, f.py, f.pz, le)) {
             if (pp.deposit) {
-                if (in) {
-                    // the segment stayed in the tet: the symmetric sample points sum to
-                    // q*w*lambda(midpoint) for the segment-cloud and Gauss-3 kernels
-                    double tx = f.px - sx, ty = f.py - sy, tz = f.pz - sz;
-                    bool tiny = sqrt(tx * tx + ty * ty + tz * tz) < 1e-15;
-                    int4 tn = rec_nodes(M, f.cur);
-                    int nd[4] = {tn.x, tn.y, tn.z, tn.w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        double lk = tiny ? lam[q] : (pp.dep_kernel == 0 ? le[q] : 0.5 * (lam[q] + le[q]));
-                        fx_red(A, nd[q], fx_from_double((qw * lk) * pp.inv_uq));
-                    }
-                } else {
-                    deposit_traj(M, S, pp, f.cur, sx, sy, sz, f.px, f.py, f.pz, A);
-                }
+                if (in)
+                    deposit_in_d(M, S, pp, f.cur, lam, le, f.px - sx, f.py - sy, f.pz - sz, A);
+                else
+                    deposit_traj(M, S, pp, f.cur, g, sx, sy, sz, f.px, f.py, f.pz, A);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) lam[q] = le[q];
             in = true;
         } else {
-            int nt = locate(M, f.px, f.py, f.pz, f.cur);
+            const int nt = locate(M, f.px, f.py, f.pz, f.cur);
             if (nt < 0) return kLost;
             f.cur = nt;
-            if (pp.deposit) deposit_traj(M, S, pp, nt, sx, sy, sz, f.px, f.py, f.pz, A);
-            in = bary64(M, nt, f.px, f.py, f.pz, lam);
+            g = load_geom(M, nt);
+            if (pp.deposit) deposit_traj(M, S, pp, nt, g, sx, sy, sz, f.px, f.py, f.pz, A);
+            in = baryg(g, f.px, f.py, f.pz, lam);
         }
         f.rem -= adt;
         ++nsub;
     }
     return f.it >= kMaxSubsteps ? kLost : kDone;
+}
+
+// The end of a particle's step in tet `tet` (< 0: inactive), with the fused MCC when COLLIDE.
+template <bool COLLIDE>
+__device__ __forceinline__ void finish_in_d(const ParticleStore& P, const SpeciesDev& S, const PushParams& pp,
+                                            int64_t i, FlightD& f, int tet, double ke, PushStats& c)
+{
+    c.ke += ke;  // updateStatistics counts every stored particle (PICCycle.cpp:941-966)
+    if (tet >= 0) {
+        c.ev |= kEvActive;
+        if (S.mcc_mode == 2) c.v2 = fmaxf(c.v2, (float)(f.vx * f.vx + f.vy * f.vy + f.vz * f.vz));  // the null-collision speed bound
+        if (COLLIDE && pp.do_mcc && S.mcc_enabled && mcc_elastic(S, pp, P.id[i], f.vx, f.vy, f.vz)) c.ev |= kEvHit;
+    }
+    P.x[i] = f.px; P.y[i] = f.py; P.z[i] = f.pz;
+    P.vx[i] = f.vx; P.vy[i] = f.vy; P.vz[i] = f.vz;
+    P.tet[i] = tet;
 }
 
 __device__ __forceinline__ void finish_d(const MeshView& M, const ParticleStore& P, const SpeciesDev& S,
@@ -177,15 +250,7 @@ __device__ __forceinline__ void finish_d(const MeshView& M, const ParticleStore&
         c.ev |= kEvLost;
         tet_out = resolve_lost(M, S, pp, L, f.px, f.py, f.pz, ke, f.cur);
     }
-    c.ke += ke;  // updateStatistics counts every stored particle (PICCycle.cpp:941-966)
-    if (tet_out >= 0) {
-        c.ev |= kEvActive;
-        if (S.mcc_mode == 2) c.v2 = fmaxf(c.v2, (float)(f.vx * f.vx + f.vy * f.vy + f.vz * f.vz));  // the null-collision speed bound
-        if (pp.do_mcc && S.mcc_enabled && mcc_elastic(S, pp, P.id[i], f.vx, f.vy, f.vz)) c.ev |= kEvHit;
-    }
-    P.x[i] = f.px; P.y[i] = f.py; P.z[i] = f.pz;
-    P.vx[i] = f.vx; P.vy[i] = f.vy; P.vz[i] = f.vz;
-    P.tet[i] = tet_out;
+    finish_in_d<true>(P, S, pp, i, f, tet_out, ke, c);
 }
 
 __device__ __forceinline__ void defer_store_d(const ParticleStore& P, const DeferList& D, unsigned slot, int64_t i,
@@ -200,53 +265,217 @@ __device__ __forceinline__ void defer_store_d(const ParticleStore& P, const Defe
     P.tet[i] = f.cur;
 }
 
-// Pass 1: every stored particle, at most kCap1 sub-steps.
-__global__ void __launch_bounds__(256) k_push_f64(const __grid_constant__ MeshView M, ParticleStore P,
-    const __grid_constant__ SpeciesDev S, const __grid_constant__ PushParams pp,
-                                                  DeferList D, ChargeAcc A,
-                                                  LedgerDev* L, unsigned long long* ke_acc, unsigned* ctr)
+// A warp's particles that left their tet in pass 1 and wait for their walk (see push_mixed.cu).
+struct WalkQueueD {
+    double sx[kWalkQueue], sy[kWalkQueue], sz[kWalkQueue], vx[kWalkQueue], vy[kWalkQueue], vz[kWalkQueue];
+    double adt[kWalkQueue], vstart[kWalkQueue];
+    uint32_t i[kWalkQueue];
+    int cur[kWalkQueue];
+};
+
+__device__ __forceinline__ WalkQueueD& walk_queue_d()
 {
-    const int64_t n = *P.count;
-    PushStats c{0.0, 0u, 0u};
+    __shared__ WalkQueueD q[kPushWarpsD];
+    return q[threadIdx.x >> 5];
+}
+
+// End of a particle's pass-1 sub-step (see end_first in push_mixed.cu).
+template <bool COLLIDE>
+__device__ __forceinline__ void end_first_d(const ParticleStore& P, const SpeciesDev& S, const PushParams& pp,
+                                            const DeferList& D, LedgerDev* L, int64_t i, FlightD& f, int st,
+                                            PushStats& c)
+{
+    double ke = 0.0;
+    if (st == kDone) {
+        const double v2 = f.vx * f.vx + f.vy * f.vy + f.vz * f.vz;
+        ke = 0.5 * S.m * v2;
+        if (!COLLIDE && pp.do_mcc && S.mcc_enabled && mcc_candidate(S, pp, P.id[i], v2)) st = kFinish;
+    }
+    const bool more = st > kDone;
+    const unsigned slot = warp_append(more, D.count);
+    if (more) {
+        f.it = st == kLost ? kItLost : (st == kFinish ? kItFinish : f.it);
+        if (slot < D.cap)
+            defer_store_d(P, D, slot, i, f);
+        else
+            atomicOr(&L->flags, (unsigned long long)kFlagDeferOverflow);  // the step fails with this flag
+    } else if (st == kDone) {
+        finish_in_d<COLLIDE>(P, S, pp, i, f, f.cur, ke, c);
+    }
+    warp_chunk_end(c);
+}
+
+// Walks m (up to 32) particles of the warp's queue from position `first` on: locate()'s walk from the
+// tet they left and the deposit in the tet they reach.  Points outside the domain are lost; those
+// the walk does not settle (a boundary face, a long walk, the tolerance band of several tets) run
+// again in pass 2, in the reference's search order.
+template <bool COLLIDE>
+__device__ __forceinline__ void walk_queued_d(const MeshView& M, const ParticleStore& P, const SpeciesDev& S,
+                                              const PushParams& pp, const DeferList& D, ChargeAcc A, LedgerDev* L,
+                                              int first, int m, PushStats& c)
+{
     const int lane = threadIdx.x & 31;
-    const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
-    warp_stats_begin();
-    for (;;) {
-        // runs of chunks, as in the mixed form
-        const int64_t b0 = (int64_t)next_chunk(ctr) * run;
-        if (b0 >= n) break;
-        for (int64_t base = b0; base < b0 + run && base < n; base += 32) {
-            const int64_t i = base + lane;
-            int st = -1;
-            FlightD f;
-            if (i < n) {
-                int t0 = P.tet[i];
-                f.vx = P.vx[i]; f.vy = P.vy[i]; f.vz = P.vz[i];
-                if (t0 <= kTetAbsorbed) {
-                    // updateStatistics sums every particle the container still holds (PICCycle.cpp:941-966)
-                    c.ke += 0.5 * S.m * (f.vx * f.vx + f.vy * f.vy + f.vz * f.vz);
-                } else {
-                    f.px = P.x[i]; f.py = P.y[i]; f.pz = P.z[i];
-                    f.vstart = sqrt(f.vx * f.vx + f.vy * f.vy + f.vz * f.vz);
-                    f.rem = pp.dt;
-                    f.it = 0;
-                    f.cur = locate(M, f.px, f.py, f.pz, t0);
-                    if (f.cur < 0) {
-                        f.cur = 0;  // result.final_element stays 0 (PICParticleAlgorithms.cpp:543,577)
-                        st = kLost;
+    const WalkQueueD& Q = walk_queue_d();
+    const int e = first + lane;
+    int st = -1;
+    int64_t i = 0;
+    FlightD f;
+    __syncwarp();
+    if (lane < m) {
+        i = Q.i[e];
+        const double adt = Q.adt[e];
+        f.vstart = Q.vstart[e];
+        f.px = fma(Q.vx[e], adt, Q.sx[e]);
+        f.py = fma(Q.vy[e], adt, Q.sy[e]);
+        f.pz = fma(Q.vz[e], adt, Q.sz[e]);
+        f.cur = Q.cur[e];
+        f.it = 1;
+        f.rem = pp.dt - adt;
+        st = kLost;
+        if (!outside_grid(M, f.px, f.py, f.pz)) {
+            st = kRedo;
+            int t = f.cur;
+            TetGeom g;
+            for (int k = 0; k < kWalkSteps; ++k) {
+                double lam[4];
+                g = load_geom(M, t);
+                const bool inside = baryg(g, f.px, f.py, f.pz, lam);
+                const double mn = fmin(fmin(lam[0], lam[1]), fmin(lam[2], lam[3]));
+                if (!(mn == mn)) break;
+                if (inside) {
+                    if (mn >= 1e-6) st = kDone;
+                    break;
+                }
+                int fc = 0;
+                double lm = lam[0];
+                if (lam[1] < lm) { lm = lam[1]; fc = 1; }
+                if (lam[2] < lm) { lm = lam[2]; fc = 2; }
+                if (lam[3] < lm) fc = 3;
+                const int nt = __ldg(reinterpret_cast<const int*>(M.geom + 16 * (int64_t)t + 12) + fc);
+                if (nt < 0) break;
+                t = nt;
+            }
+            if (st == kDone) {
+                if (pp.deposit) deposit_traj(M, S, pp, t, g, Q.sx[e], Q.sy[e], Q.sz[e], f.px, f.py, f.pz, A);
+                f.cur = t;
+                ++c.nsub;
+                if (f.rem > kMinTimeStep) st = kCapped;
+            }
+        }
+        f.vx = Q.vx[e]; f.vy = Q.vy[e]; f.vz = Q.vz[e];
+        if (st == kRedo) {  // the state of the step's start is still in the store
+            f.px = P.x[i]; f.py = P.y[i]; f.pz = P.z[i];
+            f.vx = P.vx[i]; f.vy = P.vy[i]; f.vz = P.vz[i];
+            f.rem = pp.dt;
+            f.it = 0;
+        }
+    }
+    end_first_d<COLLIDE>(P, S, pp, D, L, i, f, st, c);
+}
+
+// Pass 1 for the 32 particles [base, base + 32) of one warp: one sub-step, the leavers queued.
+template <bool COLLIDE>
+__device__ __forceinline__ void push1_warp_d(const MeshView& M, const ParticleStore& P, const SpeciesDev& S,
+                                             const PushParams& pp, const DeferList& D, ChargeAcc A, LedgerDev* L,
+                                             int64_t base, int64_t n, int& queued, PushStats& c)
+{
+    static_assert(kCap1 == 1, "pass 1 runs one sub-step");
+    const int lane = threadIdx.x & 31;
+    const int64_t i = base + lane;
+    int st = -1;
+    bool leaves = false;
+    FlightD f;
+    double adt = 0.0;
+    if (i < n) {
+        f.cur = P.tet[i];
+        f.vx = P.vx[i]; f.vy = P.vy[i]; f.vz = P.vz[i];
+        if (f.cur <= kTetAbsorbed) {
+            // updateStatistics sums every particle the container still holds (PICCycle.cpp:941-966)
+            c.ke += 0.5 * S.m * (f.vx * f.vx + f.vy * f.vy + f.vz * f.vz);
+        } else {
+            f.px = P.x[i]; f.py = P.y[i]; f.pz = P.z[i];
+            f.vstart = sqrt(f.vx * f.vx + f.vy * f.vy + f.vz * f.vz);
+            f.rem = pp.dt;
+            f.it = 0;
+            st = kRedo;  // no hint, or a hint that does not hold the point: located by pass 2
+            TetGeom g;
+            double lam[4];
+            bool in = false;
+            if (f.cur >= 0) {
+                g = load_geom(M, f.cur);
+                in = baryg(g, f.px, f.py, f.pz, lam);
+            }
+            if (in) {
+                st = kDone;
+                if (f.rem > kMinTimeStep) {
+                    const double sx = f.px, sy = f.py, sz = f.pz;
+                    adt = kick_d(M, S, pp, lam, true, f);
+                    f.px = fma(f.vx, adt, sx);
+                    f.py = fma(f.vy, adt, sy);
+                    f.pz = fma(f.vz, adt, sz);
+                    double le[4];
+                    if (baryg(g, f.px, f.py, f.pz, le)) {
+                        if (pp.deposit)
+                            deposit_in_d(M, S, pp, f.cur, lam, le, f.px - sx, f.py - sy, f.pz - sz, A);
+                        f.rem -= adt;
+                        f.it = 1;
+                        ++c.nsub;
+                        if (f.rem > kMinTimeStep) st = kCapped;
                     } else {
-                        st = advance_d(M, S, pp, f, kCap1, A, c.nsub);
+                        leaves = true;
+                        f.px = sx; f.py = sy; f.pz = sz;
                     }
                 }
             }
-            unsigned slot = warp_append(st == kCapped, D.count);
-            if (st == kCapped && slot < D.cap) {
-                defer_store_d(P, D, slot, i, f);
-            } else if (st >= 0) {
-                if (st == kCapped) st = advance_d(M, S, pp, f, 0x7fffffff, A, c.nsub);
-                finish_d(M, P, S, pp, L, i, f, st, c);
-            }
-            warp_chunk_end(c);
+        }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, leaves);
+    if (leaves) {
+        const int e = queued + __popc(m & ((1u << lane) - 1u));
+        WalkQueueD& Q = walk_queue_d();
+        Q.i[e] = (uint32_t)i;
+        Q.cur[e] = f.cur;
+        Q.sx[e] = f.px; Q.sy[e] = f.py; Q.sz[e] = f.pz;
+        Q.vx[e] = f.vx; Q.vy[e] = f.vy; Q.vz[e] = f.vz;
+        Q.adt[e] = adt;
+        Q.vstart[e] = f.vstart;
+        st = -1;
+    }
+    queued += __popc(m);
+    end_first_d<COLLIDE>(P, S, pp, D, L, i, f, st, c);
+}
+
+// Pass 1: every stored particle, one sub-step, in runs of chunks (see k_push_mixed).  Bound by the
+// latency of the records' loads at the 16 warps per SM its registers leave.  Two species of 3.5 M
+// particles at 48^3 cells, both launches: 2.24 ms with locate and a sample-by-sample deposit out of
+// line in the chunk's flow (14 of 32 threads active), 1.10 ms now; 3 blocks per SM (80 registers,
+// 346 bytes of spills) 1.25, 5 blocks of 4 warps (96 registers, 172 bytes) 1.19.
+template <bool COLLIDE>
+__global__ void __launch_bounds__(32 * kPushWarpsD, kPushBlocksD)
+    k_push_f64(const __grid_constant__ MeshView M, const __grid_constant__ ParticleStore P,
+               const __grid_constant__ SpeciesDev S, const __grid_constant__ PushParams pp, DeferList D, ChargeAcc A,
+               LedgerDev* L, unsigned long long* ke_acc, unsigned* ctr)
+{
+    const int64_t n = *P.count;
+    PushStats c{0.0, 0u, 0u};
+    const int64_t run = 32 * run_chunks(n, (int64_t)gridDim.x * (blockDim.x >> 5));
+    warp_stats_begin();
+    int64_t base = 0, end = 0;
+    int queued = 0;
+    for (bool left = true;;) {
+        if (queued >= 32 || (!left && queued > 0)) {
+            const int m = min(queued, 32);
+            queued -= m;
+            walk_queued_d<COLLIDE>(M, P, S, pp, D, A, L, queued, m, c);
+        } else if (!left) {
+            break;
+        } else if (base < end) {
+            push1_warp_d<COLLIDE>(M, P, S, pp, D, A, L, base, n, queued, c);
+            base += 32;
+        } else {
+            base = (int64_t)next_chunk(ctr) * run;
+            end = min(base + run, n);
+            left = base < n;
         }
     }
     warp_stats_flush(L, ke_acc, S.vmax);
@@ -278,7 +507,17 @@ __global__ void __launch_bounds__(256) k_push_f64_more(const __grid_constant__ M
             f.it = Din.it[e];
             f.rem = Din.rem[e];
             f.vstart = Din.vstart[e];
-            st = advance_d(M, S, pp, f, chain ? cap : 0x7fffffff, A, c.nsub);
+            const bool ends = f.it < 0;  // kItLost, kItFinish: only the end of the step is left
+            st = f.it == kItLost ? kLost : kDone;
+            if (f.it == 0) {
+                // the whole step: pass 1 did not find it in its hint, or did not settle its walk
+                f.cur = locate(M, f.px, f.py, f.pz, f.cur);
+                if (f.cur < 0) {
+                    f.cur = 0;  // result.final_element stays 0 (PICParticleAlgorithms.cpp:543,577)
+                    st = kLost;
+                }
+            }
+            if (!ends && st != kLost) st = advance_d(M, S, pp, f, chain ? cap : 0x7fffffff, A, c.nsub);
         }
         unsigned slot = chain ? warp_append(st == kCapped, Dout.count) : 0xffffffffu;
         if (st == kCapped && chain && slot < Dout.cap) {
@@ -328,7 +567,8 @@ void launch_push_f64(const MeshView& M, const ParticleStore& P, const SpeciesDev
                      const DeferList& D1, const DeferList& D2, ChargeAcc A, LedgerDev* L, unsigned long long* ke_acc,
                      unsigned* ctr, int grid, cudaStream_t st)
 {
-    k_push_f64<<<grid, 256, 0, st>>>(M, P, S, pp, D1, A, L, ke_acc, ctr);
+    auto first = pp.do_mcc && S.mcc_enabled && S.mcc_mode != 2 ? k_push_f64<true> : k_push_f64<false>;
+    first<<<grid * (8 / kPushWarpsD), 32 * kPushWarpsD, 0, st>>>(M, P, S, pp, D1, A, L, ke_acc, ctr);
     k_push_f64_more<<<grid, 256, 0, st>>>(M, P, S, pp, D1, D2, kCap2, A, L, ke_acc, ctr + 1);
     DeferList none{};
     k_push_f64_more<<<grid, 256, 0, st>>>(M, P, S, pp, D2, none, 0, A, L, ke_acc, ctr + 2);

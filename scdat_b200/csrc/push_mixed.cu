@@ -223,13 +223,6 @@ __device__ __forceinline__ void deposit_traj_f(const MeshView& M, const SpeciesD
     }
 }
 
-constexpr int kWalkQueue = 64;  // a warp's queue: up to 31 waiting and a chunk of 32 more
-// sub-step counts that mark a particle pass 1 deferred for the end of its step only
-constexpr int kItLost = -1;    // it left the mesh
-constexpr int kItFinish = -2;  // it may collide
-// ends of pass 1's sub-step besides kDone, kCapped and kLost
-enum { kFinish = 3, kRedo = 4 };  // end the step, or run the whole sub-step, in pass 2
-
 struct FlightF {
     float rx, ry, rz, vx, vy, vz;
     float rem, vstart;
