@@ -143,14 +143,22 @@ static __device__ __noinline__ int grid_lookup(const MeshView& M, double px, dou
         for (int j = lo[1]; j <= hi[1]; ++j)
             for (int i = lo[0]; i <= hi[0]; ++i) {
                 int b = i + M.gdim[0] * (j + M.gdim[1] * k);
-                int s = __ldg(M.bin_start + b), e = __ldg(M.bin_start + b + 1);
-                for (int q = s; q < e; ++q) {
-                    int t = __ldg(M.bin_tets + q);
-                    if (t >= best) break;
-                    if (bary64(M, t, px, py, pz, lam)) {
-                        best = t;
-                        break;
-                    }
+                // four candidates at a time, so that their records' loads overlap: a point in no tet
+                // (in the body) is tested against all of its bin, some 48 on a Kuhn mesh
+                const int s = __ldg(M.bin_start + b), e = __ldg(M.bin_start + b + 1);
+                for (int q = s; q < e; q += 4) {
+                    int t[4];
+                    bool in[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) t[k] = __ldg(M.bin_tets + min(q + k, e - 1));
+                    if (t[0] >= best) break;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) in[k] = bary64(M, t[k], px, py, pz, lam);
+                    const int f = in[0] ? 0 : (in[1] ? 1 : (in[2] ? 2 : (in[3] ? 3 : -1)));
+                    if (f < 0) continue;
+                    const int tf = f == 0 ? t[0] : (f == 1 ? t[1] : (f == 2 ? t[2] : t[3]));
+                    best = min(best, tf);
+                    break;
                 }
             }
     return best == 0x7fffffff ? -1 : best;
@@ -318,8 +326,9 @@ __device__ inline double see_yield(const PushParams& pp, double e_ev)
 // PICCycle::applyRuntimeBoundaryCondition + processRuntimeBoundaryEvents for one lost
 // particle (PICCycle.cpp:1221-1379).  Updates position (periodic wrap) and returns the new
 // tet code (>= 0 active, kTetAbsorbed, kTetEscaped).
+// nowhere: the search that lost the particle already found the position in no tet.
 static __device__ __noinline__ int resolve_lost(const MeshView& M, const SpeciesDev& S, const PushParams& pp, LedgerDev* L, double& px,
-                            double& py, double& pz, double ke, int hint)
+                            double& py, double& pz, double ke, int hint, bool nowhere)
 {
     int resolved = -1;
     int status = 0;  // 0 active, 1 absorbed, 2 escaped
@@ -327,7 +336,7 @@ static __device__ __noinline__ int resolve_lost(const MeshView& M, const Species
     for (int pass = 0; pass < 6 && !done; ++pass) {
         int f = detect_face(M, px, py, pz, pp.otol, pass == 0, pp.ntol);
         if (f < 0) {
-            resolved = locate(M, px, py, pz, hint);
+            resolved = pass == 0 && nowhere ? -1 : locate(M, px, py, pz, hint);
             ok = resolved >= 0;
             done = true;
             break;

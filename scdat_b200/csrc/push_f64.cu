@@ -248,7 +248,8 @@ __device__ __forceinline__ void finish_d(const MeshView& M, const ParticleStore&
     int tet_out = f.cur;
     if (st == kLost) {
         c.ev |= kEvLost;
-        tet_out = resolve_lost(M, S, pp, L, f.px, f.py, f.pz, ke, f.cur);
+        // lost before the sub-step cap: no tet holds the position
+        tet_out = resolve_lost(M, S, pp, L, f.px, f.py, f.pz, ke, f.cur, f.it < kMaxSubsteps);
     }
     finish_in_d<true>(P, S, pp, i, f, tet_out, ke, c);
 }

@@ -387,7 +387,8 @@ __device__ __forceinline__ void finish_f(const MeshView& M, const ParticleStore&
             px = f.rx; py = f.ry; pz = f.rz;
             hint = 0;
         }
-        tet_out = resolve_lost(M, S, pp, L, px, py, pz, ke, hint);
+        // lost before the sub-step cap: no tet holds the position
+        tet_out = resolve_lost(M, S, pp, L, px, py, pz, ke, hint, f.it < kMaxSubsteps);
         if (tet_out >= 0) {
             double3 o = origin(M, tet_out);
             f.rx = (float)(px - o.x); f.ry = (float)(py - o.y); f.rz = (float)(pz - o.z);
