@@ -286,13 +286,12 @@ SCDAT_API int scdat_compact(scdat_ctx* ctx);
 SCDAT_API int scdat_set_species_sort_interval(scdat_ctx* ctx, int32_t species, int32_t interval);
 
 /* Pass-1 form of one species' push in the precision form (no reference counterpart; the
- * reference pushes particle by particle).  WALKING: pass 1 gives every particle one sub-step
- * with the full relocation walk.  STAY_FIRST: pass 1 carries no walk code and completes only
- * sub-steps that end in the particle's own tet; the others go to the walking passes, which
- * redo that sub-step with the same arithmetic, so both forms give bitwise the same result.
- * STAY_FIRST is faster for a species that rarely leaves its tet (ions beside electrons of the
- * same temperature).  AUTO (default) probes STAY_FIRST every 32 pushes and keeps it while it
- * defers under a fifth of the species.  The plain FP64 form ignores the setting. */
+ * reference pushes particle by particle).  WALKING: pass 1 gives every particle one sub-step,
+ * and those that leave their tet walk to the next from a queue of their warp.  STAY_FIRST: pass 1
+ * carries no walk code and completes only sub-steps that end in the particle's own tet; the others
+ * go to the later passes, which redo that sub-step with the same arithmetic, so both forms give
+ * bitwise the same result.  AUTO (default) is WALKING, which is as fast for a species that rarely
+ * leaves its tet and faster for the others.  The plain FP64 form ignores the setting. */
 typedef enum { SCDAT_PUSH_AUTO = 0, SCDAT_PUSH_WALKING = 1, SCDAT_PUSH_STAY_FIRST = 2 } scdat_push_mode;
 SCDAT_API int scdat_set_species_push_mode(scdat_ctx* ctx, int32_t species, int32_t mode);
 

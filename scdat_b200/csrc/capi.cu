@@ -210,34 +210,6 @@ int check_flags(scdat_ctx* ctx)
 }
 
 // ---- the stages ----------------------------------------------------------------------
-// Pass-1 form of species s for this push (mixed form).  A stay-first pass 1 pays off for a
-// species of which few particles leave their tet or need more than one sub-step in a step
-// (ions beside electrons of the same temperature); for the others its deferrals cost more than
-// the walk code it drops.  Automatic choice: a stay-first probe on the first push and every
-// kStayProbe-th, then stay-first while the last probe deferred under kStayMaxFrac of the
-// species.  Both forms give bitwise the same result.
-constexpr int kStayProbe = 32;
-constexpr double kStayMaxFrac = 0.2;
-
-bool stay_first_now(scdat_ctx* ctx, int s)
-{
-    SpeciesState& S = ctx->species[s];
-    if (S.stay_pending) {  // the last stay-first push's deferral count has arrived
-        S.stay_frac = S.stay_n > 0 ? (double)ctx->h_deferred[s] / (double)S.stay_n : 1.0;
-        S.stay_pending = false;
-    }
-    bool stay;
-    if (S.push_mode == SCDAT_PUSH_WALKING)
-        stay = false;
-    else if (S.push_mode == SCDAT_PUSH_STAY_FIRST)
-        stay = true;
-    else
-        stay = S.stay_frac < 0.0 || S.pushes % kStayProbe == 0 || S.stay_frac < kStayMaxFrac;
-    ++S.pushes;
-    if (stay) S.stay_n = S.n;
-    return stay;
-}
-
 int do_push(scdat_ctx* ctx, bool do_mcc)
 {
     const int S = (int)ctx->species.size();
@@ -287,21 +259,13 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         ChargeAcc acc = ctx->mixed ? ChargeAcc{ctx->acc_l0.p + s * N, nullptr, nullptr}
                                    : ChargeAcc{ctx->acc_l0.p + s * N, ctx->acc_l1.p + s * N, ctx->acc_h.p + s * N};
         if (ctx->mixed) {
-            const bool stay = stay_first_now(ctx, s);
             launch_push_mixed(ctx->mv, P, R, sd, pp, d1, d2, acc, ctx->led.p, ctx->ke_acc.p, ctx->dcount.p + 2,
-                              grid, stay, ctx->st);
+                              grid, Ss.push_mode == SCDAT_PUSH_STAY_FIRST, ctx->st);
             if (Ss.perm_pending) {
                 Ss.perm_pending = false;
                 Ss.mix.swap(Ss.mix2);
                 Ss.tet.swap(Ss.tet2);
                 Ss.id.swap(Ss.id2);
-            }
-            if (stay) {
-                // pass 1's deferred count, read by the next push's choice (the field solve in
-                // between synchronises the stream)
-                CK(cudaMemcpyAsync(ctx->h_deferred + s, ctx->dcount.p, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                   ctx->st));
-                ctx->species[s].stay_pending = true;
             }
         } else
             launch_push_f64(ctx->mv, P, sd, pp, d1, d2, acc, ctx->led.p, ctx->ke_acc.p, ctx->dcount.p + 2,
@@ -1030,8 +994,6 @@ SCDAT_API int scdat_set_species(scdat_ctx* ctx, int32_t n_species, const scdat_s
     CK(ctx->counts.alloc((size_t)n_species));
     CK(ctx->vmax.alloc(2 * (size_t)n_species));
     CK(cudaMemsetAsync(ctx->vmax.p, 0, 2 * sizeof(unsigned) * n_species, ctx->st));
-    CK(cudaMallocHost((void**)&ctx->h_deferred, sizeof(unsigned) * n_species));
-    std::memset(ctx->h_deferred, 0, sizeof(unsigned) * n_species);
     CK(cudaMemsetAsync(ctx->counts.p, 0, sizeof(int64_t) * n_species, ctx->st));
     CK(cudaMemsetAsync(ctx->acc_l0.p, 0, sizeof(unsigned long long) * n_species * N, ctx->st));
     CK(cudaMemsetAsync(ctx->acc_l1.p, 0, sizeof(unsigned long long) * n_species * N, ctx->st));

@@ -63,14 +63,7 @@ struct SpeciesState {
     int64_t cap = 0;
     int64_t n = 0;  // host view of the stored count (updated on set/compact)
     int sort_interval = 0;  // 0: the context's params.sort_interval
-    // pass-1 form of the mixed push (scdat_set_species_push_mode) and the automatic choice's
-    // state: pushes so far, the deferred fraction of the last stay-first push (-1: none yet),
-    // the particle count of that push, and whether its count is still to be read
-    int push_mode = 0;
-    int64_t pushes = 0;
-    double stay_frac = -1.0;
-    int64_t stay_n = 0;
-    bool stay_pending = false;
+    int push_mode = 0;  // pass-1 form of the mixed push (scdat_set_species_push_mode)
     DBuf<double> x, y, z, vx, vy, vz;
     DBuf<float4> mix;  // mixed form: two float4 per particle (see ParticleStore)
     DBuf<int32_t> tet;
@@ -169,7 +162,6 @@ struct scdat_ctx {
     DBuf<int> d1it, d2it;
     DBuf<double> d1rem, d2rem, d1vs, d2vs;
     unsigned dcap = 0, d1cap = 0;
-    unsigned* h_deferred = nullptr;  // pinned: pass-1 deferred count of each species' last stay-first push
     // surface circuit of the body faces (scdat_set_surface_circuit)
     bool surface = false;
     int see_model = 0;
@@ -210,7 +202,6 @@ struct scdat_ctx {
     ~scdat_ctx()
     {
         if (st) cudaStreamSynchronize(st);
-        if (h_deferred) cudaFreeHost(h_deferred);
         for (auto* evs : {&ev_push, &ev_field, &ev_sort})
             for (auto& pr : *evs) {
                 cudaEventDestroy(pr.first);
