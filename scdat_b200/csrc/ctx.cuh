@@ -96,6 +96,37 @@ struct StageEvents {
     }
 };
 
+// Deferred-particle lists and counters of a chain of push passes, and the stream it runs on beside
+// the context's own (null: on that one).  The species' chains share no buffer, so that the later
+// passes of one, a few warps following long sub-step chains, run beside the first pass of the next.
+struct PushLane {
+    cudaStream_t st = nullptr;
+    DBuf<unsigned> count;  // defer-list counts [0, 1] and the three passes' work counters [2, 5)
+    DBuf<uint32_t> idx[2];
+    DBuf<int> it[2];
+    DBuf<double> rem[2], vs[2];
+    unsigned cap[2] = {0, 0};
+
+    // pass 1's list holds the largest species (it may defer every particle), pass 2's a quarter of
+    // it (a full one only means the overflow finishes in pass 2)
+    cudaError_t grow(int64_t particles)
+    {
+        cudaError_t e = cudaSuccess;
+        if (!count.p) e = count.alloc(5);
+        for (int l = 0; l < 2 && e == cudaSuccess; ++l) {
+            const int64_t n = (l ? particles / 4 : particles) + 4096;
+            const unsigned want = n < 0x7fffffff ? (unsigned)n : 0x7fffffffu;
+            if (want <= cap[l]) continue;
+            cap[l] = 0;
+            if ((e = idx[l].alloc(want)) == cudaSuccess && (e = it[l].alloc(want)) == cudaSuccess &&
+                (e = rem[l].alloc(want)) == cudaSuccess && (e = vs[l].alloc(want)) == cudaSuccess)
+                cap[l] = want;
+        }
+        return e;
+    }
+    DeferList list(int l) { return DeferList{count.p + l, cap[l], idx[l].p, it[l].p, rem[l].p, vs[l].p}; }
+};
+
 // One multigrid level on the device (level 0 shares the context's Poisson arrays and only
 // holds its transfers and work vectors).
 struct MgDevLevel {
@@ -156,12 +187,8 @@ struct scdat_ctx {
     DBuf<int64_t> idx64;
     DBuf<int64_t> stage_nodes;  // scdat_set_node_potentials staging
     DBuf<double> stage_vals;
-    // deferred-particle lists of the multi-pass push
-    DBuf<unsigned> dcount;
-    DBuf<uint32_t> d1idx, d2idx;
-    DBuf<int> d1it, d2it;
-    DBuf<double> d1rem, d2rem, d1vs, d2vs;
-    unsigned dcap = 0, d1cap = 0;
+    PushLane lane[2];  // the push of species 0, and of the others
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // surface circuit of the body faces (scdat_set_surface_circuit)
     bool surface = false;
     int see_model = 0;
@@ -202,6 +229,10 @@ struct scdat_ctx {
     ~scdat_ctx()
     {
         if (st) cudaStreamSynchronize(st);
+        if (lane[1].st) cudaStreamSynchronize(lane[1].st);
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_join) cudaEventDestroy(ev_join);
+        if (lane[1].st) cudaStreamDestroy(lane[1].st);
         for (auto* evs : {&ev_push, &ev_field, &ev_sort})
             for (auto& pr : *evs) {
                 cudaEventDestroy(pr.first);
