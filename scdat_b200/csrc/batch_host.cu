@@ -381,7 +381,11 @@ int after_steps(scdat_batch* b, int n)
             return rc;
         }
     }
-    return resorted ? upload_jobs(b) : SCDAT_OK;
+    if (!resorted) return SCDAT_OK;
+    // upload_jobs gathers the re-sorted stores on the contexts' streams: the next graph launch, on the
+    // batch's, waits for them
+    int rc = upload_jobs(b);
+    return rc ? rc : sync_contexts(b);
 }
 
 }  // namespace
