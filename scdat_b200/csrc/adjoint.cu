@@ -473,11 +473,11 @@ __global__ void k_adj_split(PoissonView A, const double* __restrict__ mu, double
 namespace {
 
 struct Snap {  // the state a segment is recomputed from
-    std::vector<std::unique_ptr<DBuf<double>>> d;
-    std::vector<std::unique_ptr<DBuf<int32_t>>> t;
-    DBuf<double> phi;
-    DBuf<SurfaceDev> surf;
-    DBuf<LedgerDev> led;
+    std::vector<std::unique_ptr<SBuf<double>>> d;
+    std::vector<std::unique_ptr<SBuf<int32_t>>> t;
+    SBuf<double> phi;
+    SBuf<SurfaceDev> surf;
+    SBuf<LedgerDev> led;
     int64_t steps = 0;
     double sim_time = 0.0;
 };
@@ -488,19 +488,19 @@ int snap_save(scdat_ctx* ctx, Snap& s)
     s.t.clear();
     for (auto& S : ctx->species) {
         for (DBuf<double>* a : {&S.x, &S.y, &S.z, &S.vx, &S.vy, &S.vz}) {
-            s.d.push_back(std::make_unique<DBuf<double>>());
-            if (s.d.back()->alloc(std::max<size_t>(a->n, 1)) != cudaSuccess) return SCDAT_ERR_CUDA;
+            s.d.push_back(std::make_unique<SBuf<double>>());
+            if (s.d.back()->alloc(std::max<size_t>(a->n, 1), ctx->st) != cudaSuccess) return SCDAT_ERR_CUDA;
             if (a->n) cudaMemcpyAsync(s.d.back()->p, a->p, sizeof(double) * a->n, cudaMemcpyDeviceToDevice, ctx->st);
         }
-        s.t.push_back(std::make_unique<DBuf<int32_t>>());
-        if (s.t.back()->alloc(std::max<size_t>(S.tet.n, 1)) != cudaSuccess) return SCDAT_ERR_CUDA;
+        s.t.push_back(std::make_unique<SBuf<int32_t>>());
+        if (s.t.back()->alloc(std::max<size_t>(S.tet.n, 1), ctx->st) != cudaSuccess) return SCDAT_ERR_CUDA;
         if (S.tet.n) cudaMemcpyAsync(s.t.back()->p, S.tet.p, sizeof(int32_t) * S.tet.n, cudaMemcpyDeviceToDevice, ctx->st);
     }
-    if (s.phi.alloc(ctx->hm.N) != cudaSuccess || s.led.alloc(1) != cudaSuccess) return SCDAT_ERR_CUDA;
+    if (s.phi.alloc(ctx->hm.N, ctx->st) != cudaSuccess || s.led.alloc(1, ctx->st) != cudaSuccess) return SCDAT_ERR_CUDA;
     cudaMemcpyAsync(s.phi.p, ctx->phi.p, sizeof(double) * ctx->hm.N, cudaMemcpyDeviceToDevice, ctx->st);
     cudaMemcpyAsync(s.led.p, ctx->led.p, sizeof(LedgerDev), cudaMemcpyDeviceToDevice, ctx->st);
     if (ctx->surface) {
-        if (s.surf.alloc(1) != cudaSuccess) return SCDAT_ERR_CUDA;
+        if (s.surf.alloc(1, ctx->st) != cudaSuccess) return SCDAT_ERR_CUDA;
         cudaMemcpyAsync(s.surf.p, ctx->surf.p, sizeof(SurfaceDev), cudaMemcpyDeviceToDevice, ctx->st);
     }
     s.steps = ctx->steps;
@@ -601,24 +601,24 @@ SCDAT_API int scdat_adjoint_window(scdat_ctx* ctx, const scdat_adjoint_request* 
     res->J = J;
 
     // ---- adjoint buffers
-    DBuf<double> lphi, lphid, lrho, lE, brow, mu, emit, ldq;
-    DBuf<unsigned long long> aflags;
-    ACK(lphi.alloc(N));
-    ACK(lphid.alloc(N));
-    ACK(lrho.alloc(N));
-    ACK(lE.alloc(3 * N));
-    ACK(brow.alloc(std::max(A.R, 1)));
-    ACK(mu.alloc(std::max(A.R, 1)));
-    ACK(emit.alloc(6));
-    ACK(ldq.alloc(6));
-    ACK(aflags.alloc(1));
+    SBuf<double> lphi, lphid, lrho, lE, brow, mu, emit, ldq;
+    SBuf<unsigned long long> aflags;
+    ACK(lphi.alloc(N, st));
+    ACK(lphid.alloc(N, st));
+    ACK(lrho.alloc(N, st));
+    ACK(lE.alloc(3 * N, st));
+    ACK(brow.alloc(std::max(A.R, 1), st));
+    ACK(mu.alloc(std::max(A.R, 1), st));
+    ACK(emit.alloc(6, st));
+    ACK(ldq.alloc(6, st));
+    ACK(aflags.alloc(1, st));
     ACK(cudaMemsetAsync(aflags.p, 0, sizeof(unsigned long long), st));
     ACK(cudaMemsetAsync(lE.p, 0, sizeof(double) * 3 * N, st));
-    std::vector<std::unique_ptr<DBuf<double>>> lpart;  // 6 arrays per species
+    std::vector<std::unique_ptr<SBuf<double>>> lpart;  // 6 arrays per species
     for (auto& S : ctx->species)
         for (int c = 0; c < 6; ++c) {
-            lpart.push_back(std::make_unique<DBuf<double>>());
-            ACK(lpart.back()->alloc(std::max<size_t>(S.x.n, 1)));
+            lpart.push_back(std::make_unique<SBuf<double>>());
+            ACK(lpart.back()->alloc(std::max<size_t>(S.x.n, 1), st));
             ACK(cudaMemsetAsync(lpart.back()->p, 0, sizeof(double) * std::max<size_t>(S.x.n, 1), st));
         }
     // body (bias) nodes and the surface nodes' face masks
@@ -747,16 +747,19 @@ SCDAT_API int scdat_adjoint_window(scdat_ctx* ctx, const scdat_adjoint_request* 
             if (!n) continue;
             std::vector<double> v(3 * n), l(3 * n);
             for (int c = 0; c < 3; ++c) {
-                ACK(cudaMemcpy(v.data() + c * n, ck[0].d[6 * sp + 3 + c]->p, sizeof(double) * n, cudaMemcpyDeviceToHost));
-                ACK(cudaMemcpy(l.data() + c * n, lpart[6 * sp + 3 + c]->p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+                ACK(cudaMemcpyAsync(v.data() + c * n, ck[0].d[6 * sp + 3 + c]->p, sizeof(double) * n,
+                                    cudaMemcpyDeviceToHost, st));
+                ACK(cudaMemcpyAsync(l.data() + c * n, lpart[6 * sp + 3 + c]->p, sizeof(double) * n,
+                                    cudaMemcpyDeviceToHost, st));
             }
+            ACK(cudaStreamSynchronize(st));
             for (size_t k = 0; k < 3 * n; ++k) lte += l[k] * v[k];
         }
         lte /= 2.0 * rq->te_ev;
     }
     unsigned long long fl = 0;
     if (!rc) {
-        ACK(cudaMemcpy(&fl, aflags.p, sizeof(fl), cudaMemcpyDeviceToHost));
+        ACK(cudaMemcpyAsync(&fl, aflags.p, sizeof(fl), cudaMemcpyDeviceToHost, st));
         rc = snap_load(ctx, fin);
         if (!rc) rc = do_lsq(ctx, 0.0);
         ACK(cudaStreamSynchronize(st));

@@ -352,6 +352,7 @@ int after_steps(scdat_batch* b, int n)
     std::vector<PcgScalars> o(b->ctx.size());
     BCK(cudaMemcpy(o.data(), b->sco.p, sizeof(PcgScalars) * o.size(), cudaMemcpyDeviceToHost));
     bool resorted = false;
+    // queued on every context before the host waits for any of them
     for (size_t k = 0; k < b->ctx.size(); ++k) {
         scdat_ctx* c = b->ctx[k];
         if (o[k].done < 0) {
@@ -375,12 +376,21 @@ int after_steps(scdat_batch* b, int n)
             }
             resorted = true;
         }
-        int rc = check_flags(c);
+        int rc = queue_flags(c);
         if (rc) {
             b->err = c->err;
             return rc;
         }
     }
+    int bad = SCDAT_OK;
+    for (scdat_ctx* c : b->ctx) {
+        int rc = finish_flags(c);
+        if (rc && !bad) {
+            b->err = c->err;
+            bad = rc;
+        }
+    }
+    if (bad) return bad;
     if (!resorted) return SCDAT_OK;
     // upload_jobs gathers the re-sorted stores on the contexts' streams: the next graph launch, on the
     // batch's, waits for them

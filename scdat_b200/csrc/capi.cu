@@ -193,11 +193,22 @@ PushParams push_params(const scdat_ctx* ctx, bool do_mcc)
     return pp;
 }
 
-int check_flags(scdat_ctx* ctx)
+int queue_flags(scdat_ctx* ctx)
 {
-    unsigned long long f = 0;
-    CK(cudaMemcpyAsync(&f, &ctx->led.p->flags, sizeof(f), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->flags, &ctx->led.p->flags, sizeof(ctx->pin->flags), cudaMemcpyDeviceToHost, ctx->st));
+    if (ctx->sorting)
+        CK(cudaMemcpyAsync(ctx->pin->nact, ctx->nact.p, sizeof(int64_t) * ctx->species.size(), cudaMemcpyDeviceToHost,
+                           ctx->st));
+    return SCDAT_OK;
+}
+
+int finish_flags(scdat_ctx* ctx)
+{
     CK(cudaStreamSynchronize(ctx->st));
+    for (size_t s = 0; s < ctx->species.size(); ++s)
+        if (ctx->sorting >> s & 1u) ctx->species[s].n = ctx->pin->nact[s];
+    ctx->sorting = 0;
+    const unsigned long long f = ctx->pin->flags;
     if (f & kFlagBadTet) {
         ctx->err = "device flag: invalid tet index seen";
         return SCDAT_ERR_DEVICE_FLAG;
@@ -333,8 +344,9 @@ int pcg_scalars_init(scdat_ctx* ctx, double rtol, int max_iter, double abs_thr2)
 
 int read_scalars(scdat_ctx* ctx, PcgScalars& h)
 {
-    CK(cudaMemcpyAsync(&h, ctx->sc.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->sc, ctx->sc.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    h = ctx->pin->sc;
     return SCDAT_OK;
 }
 
@@ -715,7 +727,7 @@ int do_sort(scdat_ctx* ctx, int s)
     uint32_t* kout = ctx->mixed ? S.skey.p : ctx->kout.p;
     uint32_t* vout = ctx->mixed ? S.perm.p : ctx->vout.p;
     ctx->launches += ctx->mixed ? 1 : 2;  // keys (+ the FP64 form's gather); the radix sort itself is CUB's
-    launch_sort_keys(n, S.tet.p, inactive, ctx->kin.p, ctx->vin.p, ctx->nact.p, ctx->st);
+    launch_sort_keys(n, S.tet.p, inactive, ctx->kin.p, ctx->vin.p, ctx->nact.p + s, ctx->st);
     size_t tmp = 0;
     CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, ctx->kin.p, kout, ctx->vin.p, vout, (int)n, 0, bits, ctx->st));
     if (tmp > ctx->cub_tmp.n) CK(ctx->cub_tmp.alloc(tmp));
@@ -736,7 +748,7 @@ int do_sort(scdat_ctx* ctx, int s)
         }
         in.tet = S.tet.p; in.id = S.id.p;
         out.tet = ctx->scratchi.p; out.id = ctx->scratchu.p;
-        launch_gather_store<double>(n, ctx->nact.p, perm, in, out, ctx->st);
+        launch_gather_store<double>(n, ctx->nact.p + s, perm, in, out, ctx->st);
         for (int a = 0; a < 6; ++a) da[a]->swap(ctx->shadow64[a]);
         S.tet.swap(ctx->scratchi);
         S.id.swap(ctx->scratchu);
@@ -747,12 +759,8 @@ int do_sort(scdat_ctx* ctx, int s)
         ev.commit(ctx->ev_sort);
         ctx->sorts += 1;
     }
-    int64_t act = 0;
-    CK(cudaMemcpyAsync(&act, ctx->nact.p, sizeof(act), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    S.n = act;
-    CK(cudaMemcpyAsync(ctx->counts.p + s, &S.n, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    CK(cudaMemcpyAsync(ctx->counts.p + s, ctx->nact.p + s, sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->st));
+    ctx->sorting |= 1u << s;
     return SCDAT_OK;
 }
 
@@ -961,12 +969,15 @@ int create_ctx(const scdat_mesh_desc* mesh, const scdat_params* params, scdat_ct
     CK(cudaMemsetAsync(ctx->phi.p, 0, sizeof(double) * m.N, st));
     CK(cudaMemsetAsync(ctx->E.p, 0, sizeof(double) * 3 * m.N, st));
     CK(cudaMemsetAsync(ctx->Ef.p, 0, sizeof(float) * 3 * m.N, st));
-    CK(ctx->totq.alloc(2));
-    CK(ctx->led.alloc(1));
-    CK(cudaMemsetAsync(ctx->led.p, 0, sizeof(LedgerDev), st));
-    CK(ctx->ke_acc.alloc(2));
-    CK(cudaMemsetAsync(ctx->ke_acc.p, 0, 2 * sizeof(unsigned long long), ctx->st));
-    CK(ctx->nact.alloc(1));
+    CK(ctx->stat.alloc(1));
+    CK(cudaMemsetAsync(ctx->stat.p, 0, sizeof(StatBlock), st));
+    ctx->led.p = &ctx->stat.p->led;
+    ctx->ke_acc.p = ctx->stat.p->ke;
+    ctx->totq.p = ctx->stat.p->totq;
+    CK(cudaMallocHost((void**)&ctx->pin, sizeof(HostBlock)));
+    std::memset((void*)ctx->pin, 0, sizeof(HostBlock));
+    CK(ctx->nact.alloc(16));
+    CK(cudaMemsetAsync(ctx->nact.p, 0, 16 * sizeof(int64_t), st));
     CK(cudaStreamSynchronize(st));
     return SCDAT_OK;
 }
@@ -1570,11 +1581,11 @@ SCDAT_API int scdat_get_surface_state(scdat_ctx* ctx, double* V, double* Q, doub
         ctx->err = "no surface circuit";
         return SCDAT_ERR_STATE;
     }
-    SurfaceDev h{};
-    LedgerDev l{};
-    CK(cudaMemcpyAsync(&h, ctx->surf.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&l, ctx->led.p, sizeof(l), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->surf, ctx->surf.p, sizeof(SurfaceDev), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->stat.led, ctx->led.p, sizeof(LedgerDev), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    const SurfaceDev& h = ctx->pin->surf;
+    const LedgerDev& l = ctx->pin->stat.led;
     for (int f = 0; f < 6; ++f) {
         if (V) V[f] = h.V[f];
         if (Q) Q[f] = h.Q[f];
@@ -1598,9 +1609,8 @@ SCDAT_API int scdat_push(scdat_ctx* ctx)
 {
     if (!ctx) return SCDAT_ERR_ARG;
     int rc = do_push(ctx, false);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(ctx->st));
-    return check_flags(ctx);
+    if (!rc) rc = queue_flags(ctx);
+    return rc ? rc : finish_flags(ctx);
 }
 
 SCDAT_API int scdat_solve_field(scdat_ctx* ctx)
@@ -1697,7 +1707,10 @@ SCDAT_API int scdat_compact(scdat_ctx* ctx)
         int rc = do_sort(ctx, s);
         if (rc) return rc;
     }
-    return SCDAT_OK;
+    ctx->pin->flags = 0;  // a compaction reports no flag of an earlier step
+    CK(cudaMemcpyAsync(ctx->pin->nact, ctx->nact.p, sizeof(int64_t) * ctx->species.size(), cudaMemcpyDeviceToHost,
+                       ctx->st));
+    return finish_flags(ctx);
 }
 
 SCDAT_API int scdat_step(scdat_ctx* ctx, int32_t n_steps)
@@ -1720,9 +1733,15 @@ SCDAT_API int scdat_step(scdat_ctx* ctx, int32_t n_steps)
                 if (rc) return rc;
             }
         }
+        // the next push needs the re-sorts' counts, the call's end the flags
+        if (ctx->sorting && k + 1 < n_steps) {
+            rc = queue_flags(ctx);
+            if (!rc) rc = finish_flags(ctx);
+            if (rc) return rc;
+        }
     }
-    CK(cudaStreamSynchronize(ctx->st));
-    return check_flags(ctx);
+    int rc = queue_flags(ctx);
+    return rc ? rc : finish_flags(ctx);
 }
 
 SCDAT_API int scdat_get_fields(scdat_ctx* ctx, double* rho, double* phi, double* E)
@@ -1813,9 +1832,9 @@ SCDAT_API int scdat_sample_with_derivative(scdat_ctx* const* c3, int64_t n_body,
 SCDAT_API int scdat_get_ledger(scdat_ctx* ctx, double* ledger)
 {
     if (!ctx || !ledger) return SCDAT_ERR_ARG;
-    LedgerDev h{};
-    CK(cudaMemcpyAsync(&h, ctx->led.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->stat.led, ctx->led.p, sizeof(LedgerDev), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    const LedgerDev& h = ctx->pin->stat.led;
     for (int f = 0; f < 7; ++f) {
         double* r = ledger + 8 * f;
         r[0] = fx_to_double(h.row[f][0], (long long)h.row[f][1], ctx->uq);
@@ -1881,13 +1900,10 @@ SCDAT_API int scdat_get_sort_timing(scdat_ctx* ctx, double* sort_ms, int64_t* so
 SCDAT_API int scdat_get_statistics(scdat_ctx* ctx, scdat_stats* st)
 {
     if (!ctx || !st) return SCDAT_ERR_ARG;
-    LedgerDev h{};
-    unsigned long long ke[2] = {0, 0};
-    unsigned long long tq[2] = {0, 0};
-    CK(cudaMemcpyAsync(&h, ctx->led.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(ke, ctx->ke_acc.p, sizeof(ke), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(tq, ctx->totq.p, sizeof(tq), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->pin->stat, ctx->stat.p, sizeof(StatBlock), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    const LedgerDev& h = ctx->pin->stat.led;
+    const unsigned long long *ke = ctx->pin->stat.ke, *tq = ctx->pin->stat.totq;
     std::memset(st, 0, sizeof(*st));
     st->completed_steps = ctx->steps;
     st->simulation_time = ctx->sim_time;

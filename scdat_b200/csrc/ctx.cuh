@@ -8,6 +8,7 @@
 #include "mesh_setup.h"
 #include "mg.cuh"
 #include "push.cuh"
+#include "scratch.cuh"
 #include "surface.cuh"
 
 #include <memory>
@@ -41,6 +42,11 @@ struct DBuf {
         release();
         if (count == 0) return cudaSuccess;
         cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {  // once more with the scratch pools' kept memory back
+            cudaGetLastError();
+            scratch_trim();
+            e = cudaMalloc((void**)&p, count * sizeof(T));
+        }
         if (e == cudaSuccess) n = count;
         return e;
     }
@@ -55,6 +61,24 @@ struct DBuf {
         std::swap(p, o.p);
         std::swap(n, o.n);
     }
+};
+
+// What the host reads back of a step, in one copy.
+struct StatBlock {
+    LedgerDev led;
+    unsigned long long ke[2], totq[2];
+};
+struct HostBlock {
+    StatBlock stat;
+    PcgScalars sc;
+    SurfaceDev surf;
+    int64_t nact[16];
+    unsigned long long flags;
+};
+
+template <typename T>
+struct DView {
+    T* p = nullptr;
 };
 
 struct SpeciesState {
@@ -170,20 +194,24 @@ struct scdat_ctx {
     // fields
     DBuf<double> rho, phi, E, tmp_rho;
     DBuf<float> Ef;
-    DBuf<unsigned long long> acc_l0, acc_l1, acc_h, totq;
+    DBuf<unsigned long long> acc_l0, acc_l1, acc_h;
     DBuf<unsigned> vmax;  // [2 per species]: maximum speed of the previous / current push (float bits)
     // particles
     std::vector<SpeciesState> species;
     DBuf<int64_t> counts;
-    DBuf<LedgerDev> led;
-    DBuf<unsigned long long> ke_acc;  // kinetic energy of the last push, fixed point (lo, hi)
+    DBuf<StatBlock> stat;
+    DView<LedgerDev> led;              // in stat, as the next two
+    DView<unsigned long long> ke_acc;  // kinetic energy of the last push, fixed point (lo, hi)
+    DView<unsigned long long> totq;    // total charge, fixed point (lo, hi)
+    HostBlock* pin = nullptr;          // pinned targets of the read-backs
     // sort scratch
     DBuf<uint32_t> kin, kout, vin, vout;
     DBuf<unsigned char> cub_tmp;
     DBuf<double> shadow64[6];  // re-sort targets, swapped with the store's arrays
     DBuf<int32_t> scratchi;
     DBuf<uint32_t> scratchu;
-    DBuf<int64_t> nact;
+    DBuf<int64_t> nact;  // [16] particles each species' re-sort keeps
+    unsigned sorting = 0;  // species (bits) whose re-sort is queued and whose new count is still to be read
     DBuf<int64_t> idx64;
     DBuf<int64_t> stage_nodes;  // scdat_set_node_potentials staging
     DBuf<double> stage_vals;
@@ -230,6 +258,7 @@ struct scdat_ctx {
     {
         if (st) cudaStreamSynchronize(st);
         if (lane[1].st) cudaStreamSynchronize(lane[1].st);
+        if (pin) cudaFreeHost(pin);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (lane[1].st) cudaStreamDestroy(lane[1].st);
@@ -248,8 +277,9 @@ ParticleStore store_of(scdat_ctx* ctx, int s);
 int settle_store(scdat_ctx* ctx, int s);
 SpeciesDev species_dev(const scdat_ctx* ctx, int s);
 PushParams push_params(const scdat_ctx* ctx, bool do_mcc);
-int check_flags(scdat_ctx* ctx);
-int do_sort(scdat_ctx* ctx, int s);
+int queue_flags(scdat_ctx* ctx);   // queues the read of the device flags and of the re-sorts' new counts
+int finish_flags(scdat_ctx* ctx);  // waits for it, takes the counts over and tests the flags
+int do_sort(scdat_ctx* ctx, int s);  // queued; finish_flags brings the host's count up to date
 int do_push(scdat_ctx* ctx, bool do_mcc);
 int do_surface(scdat_ctx* ctx);
 int do_solve_field(scdat_ctx* ctx);

@@ -6,6 +6,7 @@
 #include "../../include/scdat_b200.h"
 #include "pcg_csr.cuh"
 #include "pcg_group.cuh"
+#include "scratch.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -116,13 +117,12 @@ extern "C" SCDAT_API int scdat_pcg_csr(int32_t R, const int32_t* row_ptr, const 
     if (!row_ptr || !diag || !b || !x) return SCDAT_ERR_ARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int grid = 148 * 4;
-    void* base = nullptr;
-    if (cudaMalloc(&base, pcg_scratch_bytes(R, grid)) != cudaSuccess) return SCDAT_ERR_CUDA;
-    PcgScratch s = pcg_scratch_carve(base, R, grid);
+    SBuf<unsigned char> base;
+    if (base.alloc(pcg_scratch_bytes(R, grid), st) != cudaSuccess) return SCDAT_ERR_CUDA;
+    PcgScratch s = pcg_scratch_carve(base.p, R, grid);
     int it = 0;
     double rel = 0.0;
     cudaError_t e = pcg_csr_run(R, row_ptr, col, val, diag, b, x, rtol, max_iter, st, s, grid, &it, &rel);
-    cudaFree(base);
     if (e != cudaSuccess) return SCDAT_ERR_CUDA;
     if (iterations) *iterations = it;
     if (relres) *relres = rel;
