@@ -3,7 +3,7 @@
 // iteration.  Used by the single-context solves, the CSR entry points (pcg_group.cu) and, one
 // group per scenario, by the batched step (batch_field.cu).
 //
-// What bounds it: the two barriers of an iteration (4 us of 6 at 137 blocks) and the gathers'
+// What bounds it: the two barriers of an iteration (3.4 us of 5 at 137 blocks) and the gathers'
 // round trip to L2, not bandwidth.  The systems it takes (up to kCgMaxThreads * kCgRowsPerThread
 // rows per SM, 303,104 in all) fit the chip, so the two launches per iteration of the bandwidth
 // kernels (field_kern.cuh) were launch gaps and reduction tails, plus a host read every 16
@@ -44,31 +44,59 @@ struct CgGroup {
     bool dead = false;  // a barrier wait ran out: every result is void
 };
 
-// One lane posts up to 3 sums in a slot: 64-bit words of 32 data bits and the barrier's number.
+// A sum in a slot: two 64-bit words of 32 data bits and the barrier's number, so that a reader knows
+// each word by itself.
+__device__ __forceinline__ void slot_words(double v, unsigned epoch, unsigned long long (&w)[2])
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    w[0] = (b << 32) | epoch;
+    w[1] = (b & 0xffffffff00000000ull) | epoch;
+}
+
+__device__ __forceinline__ bool slot_sum(const unsigned long long (&w)[2], unsigned epoch, double& v)
+{
+    v = __longlong_as_double((long long)((w[1] & 0xffffffff00000000ull) | (w[0] >> 32)));
+    return (unsigned)w[0] == epoch && (unsigned)w[1] == epoch;
+}
+
+// One lane posts NV sums (1 to 3) in a slot.
 template <int NV>
 __device__ __forceinline__ void slot_post(unsigned long long* slot, unsigned epoch, const double (&s)[NV])
 {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const unsigned long long w = (unsigned long long)__double_as_longlong(s[k]);
-        __stcg(reinterpret_cast<ulonglong2*>(slot) + k,
-               make_ulonglong2((w << 32) | epoch, (w & 0xffffffff00000000ull) | epoch));
+    unsigned long long a[2], b[2];
+    slot_words(s[0], epoch, a);
+    slot_words(NV > 1 ? s[NV > 1 ? 1 : 0] : 0.0, epoch, b);
+    if (NV > 2) {
+        unsigned long long c[2];
+        slot_words(s[NV - 1], epoch, c);
+        __stcg(reinterpret_cast<ulonglong2*>(slot) + 2, make_ulonglong2(c[0], c[1]));
     }
+    asm volatile("st.relaxed.gpu.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(slot), "l"(a[0]), "l"(a[1]), "l"(b[0]),
+                 "l"(b[1])
+                 : "memory");
 }
 
-// Reads a slot until all its words carry the barrier's number; false when the wait ran out.
+// Reads a slot until all its words carry the barrier's number; false when the wait ran out.  One
+// 256-bit load brings two sums: 137 blocks 1.2 us for one sum, 2.2 for two with data, against 1.4 and
+// 2.8 with a 128-bit load each.
 template <int NV>
 __device__ __forceinline__ bool slot_wait(const unsigned long long* slot, unsigned epoch, double (&s)[NV])
 {
     for (unsigned polls = 0; polls < kCgMaxPolls; ++polls) {
-        bool here = true;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            unsigned long long a, b;
+        unsigned long long a[2], b[2];
+        asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(a[0]), "=l"(a[1]), "=l"(b[0]), "=l"(b[1])
+                     : "l"(slot)
+                     : "memory");
+        double second;
+        bool here = slot_sum(a, epoch, s[0]);
+        here = slot_sum(b, epoch, second) && here;
+        if (NV > 1) s[NV > 1 ? 1 : 0] = second;
+        if (NV > 2) {
+            unsigned long long c[2];
             asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
-                         : "=l"(a), "=l"(b) : "l"(slot + 2 * k) : "memory");
-            here = here && (unsigned)a == epoch && (unsigned)b == epoch;
-            s[k] = __longlong_as_double((long long)((b & 0xffffffff00000000ull) | (a >> 32)));
+                         : "=l"(c[0]), "=l"(c[1]) : "l"(slot + 4) : "memory");
+            here = slot_sum(c, epoch, s[NV - 1]) && here;
         }
         if (here) return true;
     }
@@ -81,8 +109,8 @@ __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gp
 // Group barrier that also sums: v[k] becomes the sum over every thread of the group.  A block posts
 // its part in its slot, a line of its own, and reads every other's: one trip through L2 where an
 // arrival counter takes one to arrive, one to poll and one to read the parts.  Alone, for one sum
-// without data and two sums with it, 8 blocks 0.75 / 1.2 us, 35 blocks 1.1 / 2.0, 137 blocks
-// 1.4 / 2.8 (counter and __threadfence: 2.2 / 2.6, 2.4 / 3.4, 2.7 / 3.4; slots gathered 16 at a
+// without data and two sums with it, 14 blocks 1.0 / 1.7 us, 35 blocks 1.0 / 2.0, 137 blocks
+// 1.2 / 2.2 (counter and __threadfence: 2.2 / 2.7, 2.4 / 3.4, 2.7 / 3.4; slots gathered 16 at a
 // time by a first block above 32: 1.7 / 3.3 and 2.0 / 3.7).  With DATA, everything a thread of the
 // group wrote to global memory before is visible to the others' __ldcg after.
 template <int NV, bool DATA>
@@ -403,8 +431,9 @@ __device__ __forceinline__ void cg_solve_mixed(CgGroup g, const PoissonView& P, 
 // Launch shape for groups of the given row counts on nsm SMs: one block per SM at most, as many as
 // the rows fill (a row more per thread costs an iteration 0.8 to 1.6 us, 102 more blocks 1 us of
 // barrier: 33x27x41 cells, 35k rows, 137 blocks of 256 777 us, 69 of 512 833, 35 of 512 with two
-// rows a thread 955), then more rows per thread; !ok when that does not fit.  blocks_of: blocks of
-// each group.
+// rows a thread 955), then more rows per thread, the same for every group (a batch of 8 with one row
+// a thread in its largest scenario and more in the others 7.33 ms, two in each 7.07); !ok when that
+// does not fit.  blocks_of: blocks of each group.
 CgPlan cg_plan(const int* rows, int n, int nsm, int* blocks_of);
 
 // One system: queues the solve on st.  zp: 2 R values; slots: kCgSlotBytes; results in sc (done < 0:
