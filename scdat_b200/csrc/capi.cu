@@ -13,6 +13,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -353,9 +354,27 @@ int read_scalars(scdat_ctx* ctx, PcgScalars& h)
 // Multigrid-preconditioned CG on the Dirichlet-reduced system in V's precision, from x: b, x and
 // the CG vectors r, z, p, q are R-vectors of the caller.  Blocks until the solve ends.
 template <typename V>
-int run_mgpcg(scdat_ctx* ctx, const V* b, V* x, V* r, V* z, V* p, V* q, double rtol, int max_iter, PcgScalars& h)
+const MgGroupPlan<V>& mg_group(const scdat_ctx* ctx);
+template <>
+const MgGroupPlan<float>& mg_group<float>(const scdat_ctx* ctx) { return ctx->mg_group_f; }
+template <>
+const MgGroupPlan<double>& mg_group<double>(const scdat_ctx* ctx) { return ctx->mg_group_d; }
+
+int read_group_scalars(scdat_ctx* ctx, PcgScalars& h);
+
+// zero_start: x = 0 on entry, and not read.
+template <typename V>
+int run_mgpcg(scdat_ctx* ctx, const V* b, V* x, V* r, V* z, V* p, V* q, bool zero_start, double rtol, int max_iter,
+              PcgScalars& h)
 {
     const PoissonView& A = ctx->pv;
+    const MgGroupPlan<V>& group = mg_group<V>(ctx);
+    if (group.blocks > 0) {
+        ctx->launches += 1;
+        CK(launch_mgpcg_group<V>(group, b, x, r, z, p, q, zero_start, rtol, max_iter, ctx->sc.p, ctx->part.p, ctx->st));
+        return read_group_scalars(ctx, h);
+    }
+    if (zero_start) CK(cudaMemsetAsync(x, 0, sizeof(V) * A.R, ctx->st));
     int rc = pcg_scalars_init(ctx, rtol, max_iter, 0.0);
     if (rc) return rc;
     launch_mgpcg_init<V>(A, b, x, r, ctx->sc.p, ctx->part.p, ctx->grid_red, ctx->st);
@@ -395,7 +414,7 @@ int run_pcg64(scdat_ctx* ctx, const double* bvec, double* xvec, double rtol, int
     const PoissonView& A = ctx->pv;
     if (ctx->precond == SCDAT_PRECOND_MULTIGRID) {
         PcgScalars h{};
-        int rc = run_mgpcg<double>(ctx, bvec, xvec, ctx->r.p, ctx->z.p, ctx->p.p, ctx->q.p, rtol, max_iter, h);
+        int rc = run_mgpcg<double>(ctx, bvec, xvec, ctx->r.p, ctx->z.p, ctx->p.p, ctx->q.p, false, rtol, max_iter, h);
         if (rc) return rc;
         iters = h.iter;
         relres = std::sqrt(h.rr / (h.bb > 0.0 ? h.bb : 1.0));
@@ -473,11 +492,9 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
         relres = std::sqrt(h.rr / bb);
         if (h.rr <= rtol * rtol * bb || iters >= max_iter || outer == kMaxRefinePasses) break;
         // inner FP32 solve A e = r from e = 0, to the tolerance this pass needs
-        ctx->launches += 1;
-        launch_zero_f32(R, ctx->xf.p, ctx->grid_red, ctx->st);
         if (ctx->precond == SCDAT_PRECOND_MULTIGRID) {
             PcgScalars hi{};
-            rc = run_mgpcg<float>(ctx, ctx->rf.p, ctx->xf.p, ctx->qf.p, ctx->zf.p, ctx->pf.p, ctx->pnf.p,
+            rc = run_mgpcg<float>(ctx, ctx->rf.p, ctx->xf.p, ctx->qf.p, ctx->zf.p, ctx->pf.p, ctx->pnf.p, true,
                                   inner_rtol(h.rr, bb, rtol), std::max(1, max_iter - iters), hi);
             if (rc) return rc;
             iters += hi.iter;
@@ -486,7 +503,8 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
             CK(cudaGetLastError());
             continue;
         }
-        ctx->launches += 1;
+        ctx->launches += 2;
+        launch_zero_f32(R, ctx->xf.p, ctx->grid_red, ctx->st);
         rc = pcg_scalars_init(ctx, inner_rtol(h.rr, bb, rtol), std::max(1, max_iter - iters), 0.0);
         if (rc) return rc;
         launch_pcg_init32(A, ctx->rf.p, ctx->xf.p, ctx->qf.p, ctx->zf.p, ctx->sc.p, ctx->part.p, ctx->grid_red,
@@ -516,6 +534,84 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
         launch_add_correction(R, ctx->x.p, ctx->xf.p, ctx->grid_red, ctx->st);
         CK(cudaGetLastError());
     }
+    return SCDAT_OK;
+}
+
+// The one-launch form of the hierarchy, when its finest level gives a thread kMgGroupRows rows at
+// most (303,104 on 148 SMs, what the one-launch Jacobi solve takes): 64^3 cells, FP32, 3.0 outer
+// passes, 1.28 ms against 2.09 ms by launches; beyond that four times as many threads per SM read
+// the levels.
+template <typename V>
+int setup_mg_group(scdat_ctx* ctx, const HostMg& hmg, MgGroupPlan<V>& plan, const V* cinv)
+{
+    plan = MgGroupPlan<V>{};
+    const int L = (int)hmg.lv.size(), blocks = std::min(ctx->nsm, kCgMaxGroup);
+    if (L < 2 || L > kMgMaxLevels || hmg.lv[0].R > blocks * kMgGroupThreads * kMgGroupRows) return SCDAT_OK;
+    const auto width = [](const std::vector<int32_t>& ptr) {
+        int w = 0;
+        for (size_t r = 0; r + 1 < ptr.size(); ++r) w = std::max(w, (int)(ptr[r + 1] - ptr[r]));
+        return w;
+    };
+    const auto batches = [](int w) { return (w + kMgEllBatch - 1) / kMgEllBatch * kMgEllBatch; };
+    std::vector<MgGroupLevel<V>> table((size_t)L);
+    std::vector<std::array<int, 3>> widths((size_t)L);
+    for (int l = 0; l + 1 < L; ++l) {
+        const HostMgLevel& H = hmg.lv[l];
+        widths[l] = {batches(width(l == 0 ? ctx->hps.row_ptr : H.row_ptr)), kMgEllTransfer, batches(width(H.r_ptr))};
+        if (widths[l][0] > kMgEllMax || widths[l][2] > kMgEllMax || width(H.p_ptr) > kMgEllTransfer) return SCDAT_OK;
+    }
+    constexpr bool single = sizeof(V) == sizeof(float);
+    for (int l = 0; l < L; ++l) {
+        const MgLevelDev& v = ctx->mg_plan.lv[l];
+        const MgWork& w = ctx->mg_plan.w[l];
+        MgDevLevel& D = *ctx->mgl[l];
+        MgGroupLevel<V>& g = table[l];
+        g.R = v.R;
+        g.omega = (V)v.omega;
+        g.diag = single ? (const V*)v.diagf : (const V*)v.diag;
+        g.dinv = single ? (const V*)v.dinvf : (const V*)v.dinv;
+        g.b = (V*)w.b;
+        g.xa = (V*)w.xa;
+        g.xb = (V*)w.xb;
+        g.res = (V*)w.res;
+        g.xo = (V*)w.xo;
+        if (l + 1 == L) break;  // the coarsest level is its dense inverse
+        const int rows[3] = {v.R, v.R, hmg.lv[l + 1].R};
+        const int32_t* ptr[3] = {v.row_ptr, v.p_ptr, v.r_ptr};
+        const int32_t* col[3] = {v.col, v.p_col, v.r_col};
+        EllDev<V>* out[3] = {&g.A, &g.P, &g.Rt};
+        for (int m = 0; m < 3; ++m) {
+            const size_t n = (size_t)widths[l][m] * rows[m];
+            cudaError_t e = D.ell_val[m].alloc(sizeof(V) * std::max<size_t>(n, 1));
+            if (e == cudaSuccess) e = D.ell_col[m].alloc(std::max<size_t>(n, 1));
+            if (e == cudaErrorMemoryAllocation) {  // no room for the second layout: the launched passes
+                cudaGetLastError();
+                for (int k = 0; k <= l; ++k)
+                    for (int q = 0; q < 3; ++q) {
+                        ctx->mgl[k]->ell_val[q].release();
+                        ctx->mgl[k]->ell_col[q].release();
+                    }
+                return SCDAT_OK;
+            }
+            CK(e);
+            V* ev = (V*)D.ell_val[m].p;
+            if (m == 0 && single)
+                launch_csr_to_ell<float, V>(rows[m], widths[l][m], ptr[m], col[m], v.valf, ev, D.ell_col[m].p, ctx->st);
+            else if (m == 0)
+                launch_csr_to_ell<double, V>(rows[m], widths[l][m], ptr[m], col[m], v.val, ev, D.ell_col[m].p, ctx->st);
+            else
+                launch_csr_to_ell<float, V>(rows[m], widths[l][m], ptr[m], col[m], m == 1 ? v.p_w : v.r_w, ev,
+                                            D.ell_col[m].p, ctx->st);
+            *out[m] = EllDev<V>{ev, D.ell_col[m].p, widths[l][m], rows[m]};
+        }
+    }
+    CK(cudaGetLastError());
+    CK(ctx->mg_table.upload((const unsigned char*)table.data(), sizeof(table[0]) * table.size(), ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    plan.lv = (const MgGroupLevel<V>*)ctx->mg_table.p;
+    plan.levels = L;
+    plan.cinv = cinv;
+    plan.blocks = blocks;
     return SCDAT_OK;
 }
 
@@ -617,7 +713,8 @@ int setup_multigrid(scdat_ctx* ctx)
     plan.cinv = ctx->mg_cinv.p;
     plan.cinvf = ctx->mg_cinvf.p;
     ctx->mg_plan = plan;
-    return SCDAT_OK;
+    return ctx->mixed ? setup_mg_group<float>(ctx, hmg, ctx->mg_group_f, plan.cinvf)
+                      : setup_mg_group<double>(ctx, hmg, ctx->mg_group_d, plan.cinv);
 }
 
 int do_solve_field(scdat_ctx* ctx)

@@ -7,6 +7,7 @@
 #include "field.cuh"
 #include "mesh_setup.h"
 #include "mg.cuh"
+#include "mg_group.cuh"
 #include "push.cuh"
 #include "scratch.cuh"
 #include "surface.cuh"
@@ -158,6 +159,9 @@ struct MgDevLevel {
     DBuf<double> val, diag, dinv;
     DBuf<float> valf, diagf, dinvf, p_w, r_w;
     DBuf<unsigned char> work;  // b, xa, xb, res, xo in the context's precision
+    // rows side by side for the one-launch solve: operator, prolongation, restriction
+    DBuf<unsigned char> ell_val[3];
+    DBuf<int32_t> ell_col[3];
 };
 
 struct scdat_ctx {
@@ -191,6 +195,9 @@ struct scdat_ctx {
     DBuf<double> mg_cinv;
     DBuf<float> mg_cinvf;
     MgPlan mg_plan;
+    DBuf<unsigned char> mg_table;  // MgGroupLevel of every level
+    MgGroupPlan<float> mg_group_f;   // one-launch solve (blocks == 0: none), in the context's precision
+    MgGroupPlan<double> mg_group_d;
     // fields
     DBuf<double> rho, phi, E, tmp_rho;
     DBuf<float> Ef;
