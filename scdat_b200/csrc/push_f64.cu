@@ -28,13 +28,14 @@ __device__ __forceinline__ TetGeom load_geom(const MeshView& M, int t)
     return TetGeom{{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x}, {e.y, f.x, f.y}};
 }
 
-// bary64 from a record already in registers
+// bary64 from a record already in registers.  The rounding is spelled out: left to the compiler, two
+// uses contracted differently, and a step taken up again in pass 3 could end 1 ulp from one that ran on.
 __device__ __forceinline__ bool baryg(const TetGeom& g, double px, double py, double pz, double lam[4])
 {
     const double dx = px - g.o[0], dy = py - g.o[1], dz = pz - g.o[2];
-    lam[1] = g.j[0] * dx + g.j[1] * dy + g.j[2] * dz;
-    lam[2] = g.j[3] * dx + g.j[4] * dy + g.j[5] * dz;
-    lam[3] = g.j[6] * dx + g.j[7] * dy + g.j[8] * dz;
+    lam[1] = fma(g.j[2], dz, fma(g.j[1], dy, __dmul_rn(g.j[0], dx)));
+    lam[2] = fma(g.j[5], dz, fma(g.j[4], dy, __dmul_rn(g.j[3], dx)));
+    lam[3] = fma(g.j[8], dz, fma(g.j[7], dy, __dmul_rn(g.j[6], dx)));
     lam[0] = 1.0 - lam[1] - lam[2] - lam[3];
     return bary_inside(lam);
 }
@@ -493,15 +494,22 @@ __global__ void __launch_bounds__(256) k_push_f64_more(const __grid_constant__ M
     PushStats c{0.0, 0u, 0u};
     const int lane = threadIdx.x & 31;
     const bool chain = Dout.count != nullptr;
+    int64_t base, end;
+    const bool once = list_share(n, base, end);
+    if (once && base >= n) return;
+    if (once) cap = 0x7fffffff;
     warp_stats_begin();
     for (;;) {
-        const int64_t base = (int64_t)next_chunk(ctr) * 32;
-        if (base >= n) break;
+        if (!once) {
+            base = (int64_t)next_chunk(ctr) * 32;
+            end = n;
+            if (base >= n) break;
+        }
         const int64_t e = base + lane;
         int st = -1;
         FlightD f;
         int64_t i = 0;
-        if (e < n) {
+        if (e < end) {
             i = Din.idx[e];
             f.cur = P.tet[i];
             f.px = P.x[i]; f.py = P.y[i]; f.pz = P.z[i];
@@ -529,6 +537,7 @@ __global__ void __launch_bounds__(256) k_push_f64_more(const __grid_constant__ M
             finish_d(M, P, S, pp, L, i, f, st, c);
         }
         warp_chunk_end(c);
+        if (once) break;
     }
     warp_stats_flush(L, ke_acc, S.vmax);
 }
@@ -571,6 +580,7 @@ void launch_push_f64(const MeshView& M, const ParticleStore& P, const SpeciesDev
 {
     auto first = pp.do_mcc && S.mcc_enabled && S.mcc_mode != 2 ? k_push_f64<true> : k_push_f64<false>;
     first<<<grid * (8 / kPushWarpsD), 32 * kPushWarpsD, 0, st>>>(M, P, S, pp, D1, A, L, ke_acc, ctr);
+    grid = std::min(grid, 148 * 2);  // what is resident at once
     k_push_f64_more<<<grid, 256, 0, st>>>(M, P, S, pp, D1, D2, kCap2, A, L, ke_acc, ctr + 1);
     DeferList none{};
     k_push_f64_more<<<grid, 256, 0, st>>>(M, P, S, pp, D2, none, 0, A, L, ke_acc, ctr + 2);

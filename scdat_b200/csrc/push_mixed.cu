@@ -14,8 +14,8 @@
 //
 // Sub-steps run in passes so that warps stay converged: pass 1 gives every particle at most
 // kCap1 sub-steps and appends the unfinished ones to a list, with those whose end needs more than
-// the store (lost, perhaps colliding, to be located in FP64); pass 2 gives those up to kCap2 more
-// sub-steps; pass 3 finishes the rest.  The step structure is the reference's
+// the store (lost, perhaps colliding, to be located in FP64); pass 2 ends a short list's steps and
+// gives those of a long one up to kCap2 more sub-steps; pass 3 finishes the rest.  The step structure is the reference's
 // CrossTetrahedron::integrateTrajectory (PICParticleAlgorithms.cpp:536-740).
 #include "batch.cuh"
 #include "push.cuh"
@@ -693,7 +693,7 @@ __device__ __forceinline__ void push1_stay_warp(const MeshView& M, const Particl
     end_first<COLLIDE>(P, S, pp, D, L, i, f, st, c);
 }
 
-// Passes 2 and 3 for entries [base, base + 32) of list Din (up to `cap` sub-steps, then
+// Passes 2 and 3 for entries [base, n), 32 at most, of list Din (up to `cap` sub-steps, then
 // append to Dout; with Dout.count == nullptr the particles run to the end).
 __device__ __forceinline__ void push_more_warp(const MeshView& M, const ParticleStore& P, const SpeciesDev& S,
                                                const PushParams& pp, const DeferList& Din, const DeferList& Dout,
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_stay(const __grid_constan
     warp_stats_flush(L, ke_acc, S.vmax);
 }
 
-// Passes 2 and 3, 4 blocks of 256 per SM (64 registers; the four launches of a step at 64^3 cells,
+// Passes 2 and 3 (list_share), 4 blocks of 256 per SM (64 registers; the four launches of a step at 64^3 cells,
 // 64 ppc: 4 blocks 598 us, 3 blocks 610, 5 blocks 641).
 __global__ void __launch_bounds__(256, 4) k_push_mixed_more(const __grid_constant__ MeshView M, ParticleStore P,
                                                          const __grid_constant__ SpeciesDev S,
@@ -815,18 +815,27 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_more(const __grid_constan
     const int64_t n = (int64_t)min(*Din.count, Din.cap);
     if (n == 0) return;  // 3 us; every warp's first atomic on the work counter alone takes 9
     PushStats c{0.0, 0u, 0u};
+    int64_t base, end;
+    const bool once = list_share(n, base, end);
+    if (once && base >= n) return;
+    if (once) cap = 0x7fffffff;
     warp_stats_begin();
     for (;;) {
-        const int64_t base = (int64_t)next_chunk(ctr) * 32;
-        if (base >= n) break;
-        push_more_warp(M, P, S, pp, Din, Dout, cap, A, L, base, n, c);
+        if (!once) {
+            base = (int64_t)next_chunk(ctr) * 32;
+            end = n;
+            if (base >= n) break;
+        }
+        push_more_warp(M, P, S, pp, Din, Dout, cap, A, L, base, end, c);
+        if (once) break;
     }
     warp_stats_flush(L, ke_acc, S.vmax);
 }
 
 // ---- batched step: all (scenario, species) jobs in one launch per pass -----------------
-// pre[njobs + 1]: 32-particle chunks per unit, chosen over all jobs (run_chunks; warps: those of
-// the pass's launch).
+// pre[njobs + 1]: pass 1's 32-particle chunks per unit, chosen over all jobs (run_chunks; warps: those
+// of the pass's launch); later passes' entries per unit when one round takes all lists (see
+// list_share; the unit is then walked to its end), else 0 for 32.
 __global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int pass, int64_t warps,
                                int64_t* __restrict__ pre, unsigned* __restrict__ ctr)
 {
@@ -846,8 +855,9 @@ __global__ void k_batch_prefix(const PushJob* __restrict__ jobs, int njobs, int 
     if (threadIdx.x == 0) {
         int64_t total = 0;
         for (int j = 0; j < njobs; ++j) total += cnt[j];
-        const int run = pass == 1 ? run_chunks(total, warps) : 1;
-        const int64_t unit = 32 * run;  // particles per counter value
+        const int64_t per = (total + warps - 1) / warps;
+        const int64_t run = pass == 1 ? run_chunks(total, warps) : per <= 32 ? per : 0;
+        const int64_t unit = pass == 1 ? 32 * run : run > 0 ? run : 32;  // particles per counter value
         int64_t a = 0;
         for (int j = 0; j < njobs; ++j) {
             pre[j] = a;
@@ -927,7 +937,7 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __re
     __shared__ int64_t spre[kMaxBatchJobs + 1];
     for (int j = threadIdx.x; j <= njobs; j += blockDim.x) spre[j] = pre[j];
     __syncthreads();
-    const int64_t total = spre[njobs];
+    const int64_t total = spre[njobs], per = pre[njobs + 1], unit = per > 0 ? per : 32;
     PushStats c{0.0, 0u, 0u};
     warp_stats_begin();
     int cur = -1;
@@ -940,13 +950,14 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __re
             cur = j;
         }
         const PushJob& J = jobs[cur];
-        const int64_t base = (g - spre[cur]) * 32;
+        const int64_t base = (g - spre[cur]) * unit;
         if (PASS == 2) {
             const int64_t n = min((int64_t)*J.D1.count, (int64_t)J.D1.cap);
-            push_more_warp(J.M, J.P, J.S, J.pp, J.D1, J.D2, kCap2, J.A, J.L, base, n, c);
+            push_more_warp(J.M, J.P, J.S, J.pp, J.D1, J.D2, per > 0 ? 0x7fffffff : kCap2, J.A, J.L, base,
+                           min(base + unit, n), c);
         } else {
             const int64_t n = min((int64_t)*J.D2.count, (int64_t)J.D2.cap);
-            push_more_warp(J.M, J.P, J.S, J.pp, J.D2, DeferList{}, 0, J.A, J.L, base, n, c);
+            push_more_warp(J.M, J.P, J.S, J.pp, J.D2, DeferList{}, 0, J.A, J.L, base, min(base + unit, n), c);
         }
     }
     if (cur >= 0) warp_stats_flush(jobs[cur].L, jobs[cur].ke_acc, jobs[cur].S.vmax);
@@ -1032,6 +1043,7 @@ void launch_push_mixed(const MeshView& M, const ParticleStore& P, const SortedSo
     auto first = stay_first ? (collide ? k_push_mixed_stay<true> : k_push_mixed_stay<false>)
                             : (collide ? k_push_mixed<true> : k_push_mixed<false>);
     first<<<grid, 256, 0, st>>>(M, P, R, S, pp, D1, A, L, ke_acc, ctr);
+    grid = std::min(grid, 148 * 4);  // what is resident at once
     k_push_mixed_more<<<grid, 256, 0, st>>>(M, P, S, pp, D1, D2, kCap2, A, L, ke_acc, ctr + 1);
     DeferList none{};
     k_push_mixed_more<<<grid, 256, 0, st>>>(M, P, S, pp, D2, none, 0, A, L, ke_acc, ctr + 2);
