@@ -1,6 +1,8 @@
 // pcg_group.cu -- launches of the one-launch Jacobi-PCG (pcg_group.cuh) on a single system.
 #include "pcg_group.cuh"
 
+#include <algorithm>
+
 namespace scdat {
 
 namespace {
@@ -41,8 +43,11 @@ CgPlan cg_plan(const int* rows, int n, int nsm, int* blocks_of)
 {
     CgPlan plan;
     if (nsm > kCgMaxGroup) nsm = kCgMaxGroup;
+    int most = 0;
+    for (int k = 0; k < n; ++k) most = std::max(most, rows[k]);
+    const bool one_block = most > 256 && most <= kCgMaxThreads;
     for (int kr = 1; kr <= kCgRowsPerThread; ++kr)
-        for (int threads = kr == 1 ? 256 : kCgMaxThreads; threads <= kCgMaxThreads; threads *= 2) {
+        for (int threads = kr == 1 && !one_block ? 256 : kCgMaxThreads; threads <= kCgMaxThreads; threads *= 2) {
             int64_t blocks = 0;
             for (int k = 0; k < n; ++k) {
                 const int64_t per = (int64_t)threads * kr;

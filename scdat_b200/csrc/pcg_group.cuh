@@ -112,7 +112,7 @@ __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gp
 // without data and two sums with it, 14 blocks 1.0 / 1.7 us, 35 blocks 1.0 / 2.0, 137 blocks
 // 1.2 / 2.2 (counter and __threadfence: 2.2 / 2.7, 2.4 / 3.4, 2.7 / 3.4; slots gathered 16 at a
 // time by a first block above 32: 1.7 / 3.3 and 2.0 / 3.7).  With DATA, everything a thread of the
-// group wrote to global memory before is visible to the others' __ldcg after.
+// group wrote to global memory before is visible to the others after.
 template <int NV, bool DATA>
 __device__ __forceinline__ void group_sync_sum(CgGroup& g, double (&v)[NV])
 {
@@ -245,7 +245,9 @@ __device__ __forceinline__ double as_stored(double v)
 // The CG loop on V vectors, carried as doubles that hold V values.  In: x, r, z of this thread's
 // rows, with (z, 0) in zp (a DATA barrier has passed since).  zp holds each row's z and last
 // direction side by side, so the mat-vec builds a column's new direction z + beta p from one load;
-// it is written once an iteration, between the two barriers the mat-vec does not touch it in.
+// it is written once an iteration, between the two barriers the mat-vec does not touch it in, and read
+// through L1, which the second barrier's fences empty (FP64 field stage of 117 rows 95 -> 79 us,
+// 33x27x41 cells 569 -> 558; a batch of 8 with two rows a thread, four steps, 7.01 -> 6.94 ms).
 struct CgScalars {
     double rz, rz_prev, rr, thr2;
     int iter, max_iter;
@@ -269,7 +271,7 @@ __device__ __forceinline__ void cg_iterate(CgGroup& g, const CgRows<V, KR>& A, c
             if (A.row[j] < 0) continue;
             const double pi = z[j] + beta * p[j];
             const double s = cg_row_apply(A, j, diag[j] * pi, [&](int c0) {
-                const double2 n = __ldcg(zp + c0);
+                const double2 n = zp[c0];  // by L1: a block's rows are neighbours
                 return n.x + beta * n.y;
             });
             p[j] = as_stored<V>(pi);
@@ -432,8 +434,10 @@ __device__ __forceinline__ void cg_solve_mixed(CgGroup g, const PoissonView& P, 
 // the rows fill (a row more per thread costs an iteration 0.8 to 1.6 us, 102 more blocks 1 us of
 // barrier: 33x27x41 cells, 35k rows, 137 blocks of 256 777 us, 69 of 512 833, 35 of 512 with two
 // rows a thread 955), then more rows per thread, the same for every group (a batch of 8 with one row
-// a thread in its largest scenario and more in the others 7.33 ms, two in each 7.07); !ok when that
-// does not fit.  blocks_of: blocks of each group.
+// a thread in its largest scenario and more in the others 7.33 ms, two in each 7.07); up to 512 rows one
+// block, whose barriers stay in the SM (FP64 field stage of 335 rows 151 -> 108 us, 504 rows 153 -> 127;
+// 992 rows two a thread in one block 199, in four blocks 177); !ok when that does not fit.
+// blocks_of: blocks of each group.
 CgPlan cg_plan(const int* rows, int n, int nsm, int* blocks_of);
 
 // One system: queues the solve on st.  zp: 2 R values; slots: kCgSlotBytes; results in sc (done < 0:

@@ -1,4 +1,4 @@
-"""The one-launch Jacobi-CG at the edges of its launch shapes: one row, a block's rows and one more,
+"""The one-launch Jacobi-CG at the edges of its launch shapes: one row, a block's rows and one more (256 or 512),
 one block per SM (148 x 256, 148 x 512) and one row more, two to four rows a thread, its largest
 system and the first of the two-launch form; rows without entries and rows longer than the part of
 the matrix that shared memory keeps.  Oracle: the solution the right-hand side was made from, in
@@ -35,7 +35,7 @@ def _system(R, rng):
     return np.cumsum(ptr).astype(np.int32), cols.astype(np.int32), vals, diag, rows
 
 
-@pytest.mark.parametrize("R", (1, 2, 255, 256, 257, 4097, SM * 256, SM * 256 + 1, SM * 512 + 1, SM * 1024 + 1,
+@pytest.mark.parametrize("R", (1, 2, 255, 256, 257, 512, 513, 4097, SM * 256, SM * 256 + 1, SM * 512 + 1, SM * 1024 + 1,
                                SM * 1536 + 1, SM * 2048, SM * 2048 + 1))
 def test_solution_at_the_edges_of_the_launch_shapes(lib, R):
     rng = np.random.default_rng(R)
