@@ -57,7 +57,7 @@ void launch_gather_mixed(int64_t n, const int64_t* active, const uint32_t* perm,
                          uint32_t nohint_key, const float4* in_mix, const uint32_t* in_id, float4* out_mix,
                          int32_t* out_tet, uint32_t* out_id, cudaStream_t st);
 void launch_scatter_values(int64_t n, const int64_t* idx, const double* v, double* dst, cudaStream_t st);
-void launch_rotate_vmax(int S, unsigned* v, cudaStream_t st);
+void launch_push_begin(const PushBegin& b, cudaStream_t st);
 }  // namespace scdat
 
 using namespace scdat;
@@ -230,15 +230,12 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         return SCDAT_ERR_STATE;
     }
     const int64_t N = ctx->hm.N;
-    CK(cudaMemsetAsync(ctx->acc_l0.p, 0, sizeof(unsigned long long) * S * N, ctx->st));
-    if (!ctx->mixed) {  // the precision form accumulates one word per node (fx_red_word)
-        CK(cudaMemsetAsync(ctx->acc_l1.p, 0, sizeof(unsigned long long) * S * N, ctx->st));
-        CK(cudaMemsetAsync(ctx->acc_h.p, 0, sizeof(unsigned long long) * S * N, ctx->st));
-    }
-    CK(cudaMemsetAsync(ctx->ke_acc.p, 0, 2 * sizeof(unsigned long long), ctx->st));
-    CK(cudaMemsetAsync(&ctx->led.p->active, 0, sizeof(unsigned long long), ctx->st));
     ++ctx->launches;
-    launch_rotate_vmax(S, ctx->vmax.p, ctx->st);
+    // the precision form accumulates one word per node (fx_red_word)
+    launch_push_begin(PushBegin{{ctx->acc_l0.p, ctx->mixed ? nullptr : ctx->acc_l1.p, ctx->mixed ? nullptr : ctx->acc_h.p},
+                                S * N, ctx->ke_acc.p, ctx->totq.p, &ctx->led.p->active,
+                                {ctx->lane[0].count.p, ctx->lane[1].count.p}, ctx->vmax.p, S},
+                      ctx->st);
     PushParams pp = push_params(ctx, do_mcc);
     StageEvents ev;
     if (ctx->timing) {
@@ -275,7 +272,7 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         SpeciesDev sd = species_dev(ctx, s);
         // no more blocks than the species has chunks for (8 warps a block, a chunk each), but one per SM
         const int grid = (int)std::max<int64_t>(ctx->nsm, std::min<int64_t>(ctx->grid_push, (Ss.n + 255) / 256));
-        CK(cudaMemsetAsync(lane.count.p, 0, 5 * sizeof(unsigned), st));
+        if (s > 1) CK(cudaMemsetAsync(lane.count.p, 0, kLaneCounts * sizeof(unsigned), st));  // the lane's next species
         const DeferList d1 = lane.list(0), d2 = lane.list(1);
         ctx->launches += 3;
         ChargeAcc acc = ctx->mixed ? ChargeAcc{ctx->acc_l0.p + s * N, nullptr, nullptr}
@@ -302,7 +299,6 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         ev.commit(ctx->ev_push);
         ctx->push_launches += 1;
     }
-    CK(cudaMemsetAsync(ctx->totq.p, 0, sizeof(unsigned long long) * 2, ctx->st));
     ++ctx->launches;
     launch_finalize_rho(N, S, ctx->acc_l0.p, ctx->mixed ? nullptr : ctx->acc_l1.p, ctx->mixed ? nullptr : ctx->acc_h.p,
                         ctx->uq, ctx->rho.p, ctx->totq.p,
@@ -727,9 +723,9 @@ int do_solve_field(scdat_ctx* ctx)
         CK(cudaEventRecord(ev.e0, ctx->st));
     }
     if (A.R > 0) {
-        ctx->launches += 3;
-        launch_gather_rows(A, ctx->phi.p, ctx->x.p, ctx->grid_red, ctx->st);
-        launch_rhs(A, ctx->rho.p, ctx->phi.p, (double)ctx->prm.poisson_charge_sign, ctx->b.p, ctx->grid_red, ctx->st);
+        ctx->launches += 2;
+        launch_field_begin(A, ctx->rho.p, ctx->phi.p, (double)ctx->prm.poisson_charge_sign, ctx->b.p, ctx->x.p,
+                           ctx->grid_red, ctx->st);
         CK(cudaGetLastError());
         int it = 0;
         double rel = 0.0;

@@ -137,7 +137,7 @@ struct PushLane {
     cudaError_t grow(int64_t particles)
     {
         cudaError_t e = cudaSuccess;
-        if (!count.p) e = count.alloc(5);
+        if (!count.p) e = count.alloc(kLaneCounts);
         for (int l = 0; l < 2 && e == cudaSuccess; ++l) {
             const int64_t n = (l ? particles / 4 : particles) + 4096;
             const unsigned want = n < 0x7fffffff ? (unsigned)n : 0x7fffffffu;

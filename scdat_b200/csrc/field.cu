@@ -27,15 +27,12 @@ __global__ void k_species_rho(int64_t N, const unsigned long long* __restrict__ 
     k_species_rho_body(N, l0, l1, h, unit, out, Grid{blockIdx.x, gridDim.x});
 }
 
-__global__ void k_rhs(PoissonView A, const double* __restrict__ rho, const double* __restrict__ phi, double sign,
-                      double* __restrict__ b)
-{
-    k_rhs_body(A, rho, phi, sign, b, Grid{blockIdx.x, gridDim.x});
-}
-
-__global__ void k_gather_rows(PoissonView A, const double* __restrict__ phi, double* __restrict__ x)
+// the start and the right-hand side of a solve
+__global__ void k_field_begin(PoissonView A, const double* __restrict__ rho, const double* __restrict__ phi, double sign,
+                              double* __restrict__ b, double* __restrict__ x)
 {
     k_gather_rows_body(A, phi, x, Grid{blockIdx.x, gridDim.x});
+    k_rhs_body(A, rho, phi, sign, b, Grid{blockIdx.x, gridDim.x});
 }
 
 __global__ void k_scatter_rows(PoissonView A, const double* __restrict__ x, double* __restrict__ phi)
@@ -108,15 +105,10 @@ void launch_species_rho(int64_t N, const unsigned long long* l0, const unsigned 
     k_species_rho<<<grid, 256, 0, st>>>(N, l0, l1, h, unit, out);
 }
 
-void launch_rhs(const PoissonView& A, const double* rho, const double* phi, double sign, double* b, int grid,
-                cudaStream_t st)
+void launch_field_begin(const PoissonView& A, const double* rho, const double* phi, double sign, double* b, double* x,
+                        int grid, cudaStream_t st)
 {
-    k_rhs<<<grid, 256, 0, st>>>(A, rho, phi, sign, b);
-}
-
-void launch_gather_rows(const PoissonView& A, const double* phi, double* x, int grid, cudaStream_t st)
-{
-    k_gather_rows<<<grid, 256, 0, st>>>(A, phi, x);
+    k_field_begin<<<grid, 256, 0, st>>>(A, rho, phi, sign, b, x);
 }
 
 void launch_scatter_rows(const PoissonView& A, const double* x, double* phi, int grid, cudaStream_t st)

@@ -51,9 +51,8 @@ void launch_finalize_rho(int64_t N, int S, const unsigned long long* l0, const u
                          unsigned long long* thi, int grid, cudaStream_t st);
 void launch_species_rho(int64_t N, const unsigned long long* l0, const unsigned long long* l1,
                         const unsigned long long* h, double unit, double* out, int grid, cudaStream_t st);
-void launch_rhs(const PoissonView& A, const double* rho, const double* phi, double sign, double* b, int grid,
-                cudaStream_t st);
-void launch_gather_rows(const PoissonView& A, const double* phi, double* x, int grid, cudaStream_t st);
+void launch_field_begin(const PoissonView& A, const double* rho, const double* phi, double sign, double* b, double* x,
+                        int grid, cudaStream_t st);
 void launch_scatter_rows(const PoissonView& A, const double* x, double* phi, int grid, cudaStream_t st);
 void launch_lsq(int64_t N, const double* xyz, const int32_t* gptr, const int32_t* gcol, const double* phi, double reg,
                 double* E, float* Ef, unsigned long long* flags, int grid, cudaStream_t st);

@@ -654,6 +654,19 @@ __device__ __forceinline__ unsigned warp_append(bool want, unsigned* cnt)
     return base + (unsigned)__popc(m & ((1u << lane) - 1u));
 }
 
+// What a push accumulates into and starts from zero: charge words per node and species (acc, null where
+// the form has none), kinetic energy, total charge, the ledger's count of active particles, the lanes'
+// list counts and work counters (null: not there); and the species' maximum speeds, which rotate.
+constexpr int kLaneCounts = 5;
+struct PushBegin {
+    unsigned long long* acc[3];
+    int64_t words;
+    unsigned long long *ke, *totq, *active;  // ke[2], totq[2]
+    unsigned* count[2];
+    unsigned* vmax;
+    int species;
+};
+
 constexpr int kCap1 = 1;   // sub-steps every particle gets in pass 1 (1, 2, 4: 45.6, 46.1, 47.0 ms at 128^3)
 constexpr int kCap2 = 16;  // further sub-steps in pass 2 of a long list (list_share); pass 3 runs to the end
 

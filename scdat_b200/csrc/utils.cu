@@ -104,17 +104,30 @@ __global__ void k_scatter_values(int64_t n, const int64_t* __restrict__ idx, con
         dst[idx[i]] = v[i];
 }
 
-// Start of a push: each species' maximum speed of the previous push becomes the one the
-// null-collision MCC uses ([2s] <- [2s+1]), and the current slot starts from zero.
-__global__ void k_rotate_vmax(int S, unsigned* v)
+// Start of a push: all it accumulates into from zero, in one launch (a memset each, seven to nine of
+// them, took 2 us apiece in line); each species' maximum speed of the previous push becomes the one
+// the null-collision MCC uses ([2s] <- [2s+1]), and the current slot starts from zero.
+__global__ void k_push_begin(const __grid_constant__ PushBegin b)
 {
-    for (int s = threadIdx.x; s < S; s += blockDim.x) {
-        v[2 * s] = v[2 * s + 1];
-        v[2 * s + 1] = 0u;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int a = 0; a < 3; ++a)
+        if (b.acc[a])
+            for (int64_t w = t; w < b.words; w += step) b.acc[a][w] = 0ull;
+    if (t < 2) b.ke[t] = b.totq[t] = 0ull;
+    if (t == 2) *b.active = 0ull;
+    for (int l = 0; l < 2; ++l)
+        if (b.count[l] && t < kLaneCounts) b.count[l][t] = 0u;
+    for (int64_t s = t; s < b.species; s += step) {
+        b.vmax[2 * s] = b.vmax[2 * s + 1];
+        b.vmax[2 * s + 1] = 0u;
     }
 }
 
-void launch_rotate_vmax(int S, unsigned* v, cudaStream_t st) { k_rotate_vmax<<<1, 32, 0, st>>>(S, v); }
+void launch_push_begin(const PushBegin& b, cudaStream_t st)
+{
+    const int grid = (int)std::min<int64_t>((b.words + 255) / 256, 148 * 8);
+    k_push_begin<<<std::max(grid, 1), 256, 0, st>>>(b);
+}
 
 void launch_scatter_values(int64_t n, const int64_t* idx, const double* v, double* dst, cudaStream_t st)
 {
