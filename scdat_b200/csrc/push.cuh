@@ -668,6 +668,10 @@ struct PushBegin {
 };
 
 constexpr int kCap1 = 1;   // sub-steps every particle gets in pass 1 (1, 2, 4: 45.6, 46.1, 47.0 ms at 128^3)
-constexpr int kCap2 = 16;  // further sub-steps in pass 2 of a long list (list_share); pass 3 runs to the end
+// Further sub-steps in pass 2 of a long list (list_share); pass 3 runs to the end.  Pass 3 has few
+// entries, so it costs its longest walk alone: more of them end in pass 2.  Push per step with 16, 64
+// and no cap: mixed 64^3 cells, 64 ppc 2499, 2462, 2446 us; FP64 48^3 1305, 1271, 1270; 1.4 M particles
+// at 34 sub-steps each, mixed 1589, 1175, 1308, FP64 2270, 1912, 2074.
+constexpr int kCap2 = 64;
 
 }  // namespace scdat
