@@ -331,10 +331,10 @@ SCDAT_API int scdat_get_statistics(scdat_ctx* ctx, scdat_stats* st);
  * time) ----
  * A batch advances many independent contexts (each with its own mesh, species, particles and
  * potentials, all created with SCDAT_PREC_MIXED) together: every push pass is one launch over
- * all (scenario, species) pairs, the field solve one launch per kernel over all scenarios with
- * per-scenario convergence, and the whole step is captured once as a CUDA graph whose solver
- * loops are conditional nodes.  The contexts stay valid for every query (scdat_get_*); step
- * them only through the batch while it exists. */
+ * all (scenario, species) pairs, the field solve one launch over all scenarios with per-scenario
+ * convergence (one per kernel, in loops on the device, when the scenarios' rows do not fit the
+ * SMs at once), and the whole step is captured once as a CUDA graph.  The contexts stay valid for
+ * every query (scdat_get_*); step them only through the batch while it exists. */
 typedef struct scdat_batch scdat_batch;
 typedef struct {
     int32_t push_blocks_per_sm;   /* grid of the push launches, in blocks of 256 per SM (default 4) */
@@ -438,7 +438,8 @@ SCDAT_API int scdat_get_sort_timing(scdat_ctx* ctx, double* sort_ms, int64_t* so
  * its diagonal in diag[r]; x is the start vector on entry and the solution on return; the
  * solve stops when ||r|| <= rtol*||b|| or after max_iter iterations (SCDAT_ERR_NOT_CONVERGED,
  * x kept).  stream is a cudaStream_t (NULL: the default stream); the call blocks until the
- * solve ends.  Scratch device memory (6 vectors of R doubles) is allocated and freed inside. */
+ * solve ends.  Scratch device memory (6 vectors of R doubles) comes from a memory pool of the
+ * library's own, which keeps up to 128 MB per device between calls. */
 SCDAT_API int scdat_pcg_csr(int32_t R, const int32_t* row_ptr, const int32_t* col, const double* val,
                             const double* diag, const double* b, double* x, double rtol, int32_t max_iter,
                             void* stream, int32_t* iterations, double* relres);

@@ -1,8 +1,9 @@
 // batch_field.cu -- the field half of the batched step: charge finalisation, right-hand side,
-// the mixed-form solve (FP32-SpMV PCG inside FP64 refinement) and the nodal field, each one
-// launch over all scenarios.  Every block runs a single-scenario body (field_kern.cuh) on
-// its scenario's arrays; the loop control of the solve is on the device (per-scenario
-// convergence flags, and CUDA-graph conditional handles when the step is captured).
+// the mixed-form solve (FP32 PCG inside FP64 refinement) and the nodal field, each one launch over
+// all scenarios.  Every block runs a single-scenario body (field_kern.cuh, the solve
+// pcg_group.cuh) on its scenario's arrays.  Scenarios whose rows do not fit the SMs at once are
+// solved by one launch per kernel, the loop control on the device (per-scenario convergence flags,
+// and CUDA-graph conditional handles when the step is captured).
 #include "batch.cuh"
 #include "field_kern.cuh"
 #include "pcg_group.cuh"

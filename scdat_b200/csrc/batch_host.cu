@@ -1,11 +1,13 @@
 // batch_host.cu -- scdat_batch: many independent scenarios (each a scdat_ctx with its own mesh,
 // species and particles) advanced together.  One step is: zero the accumulators, three push
 // passes each launched once over every (scenario, species) job, charge finalisation and
-// right-hand side over every scenario, the mixed-form field solve with its refinement and
-// PCG loops controlled on the device, then potentials, nodal field and tet records.  The step
-// is captured once as a CUDA graph whose two loops are conditional WHILE nodes, so a step is
-// one graph launch with no host round trip; scdat_batch_tuning chooses the launch shapes and
-// scdat_batch_autotune times the candidates on the live batch.
+// right-hand side over every scenario, the mixed-form field solve, then potentials, nodal field and
+// tet records.  The solve is one cooperative launch, a group of blocks per scenario (pcg_group.cuh);
+// scenarios too large for that get one launch per kernel with the refinement and PCG loops controlled
+// on the device.  The step is captured once as a CUDA graph (whose loops, in that second case, are
+// conditional WHILE nodes), so a step is one graph launch with no host round trip;
+// scdat_batch_tuning chooses the launch shapes and scdat_batch_autotune times the candidates on the
+// live batch.
 #include "batch.cuh"
 #include "ctx.cuh"
 
