@@ -534,9 +534,10 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
 }
 
 // The one-launch form of the hierarchy, when its finest level gives a thread kMgGroupRows rows at
-// most (303,104 on 148 SMs, what the one-launch Jacobi solve takes): 64^3 cells, FP32, 3.0 outer
-// passes, 1.28 ms against 2.09 ms by launches; beyond that four times as many threads per SM read
-// the levels.
+// most (2,424,832 on 148 SMs).  Field stage, launches against one launch: FP32 16^3 cells 0.81 -> 0.45
+// ms, 64^3 2.18 -> 1.28, 96^3 4.54 -> 3.73, 128^3 (27 rows a thread) 3.46 -> 3.23; FP64 64^3 2.51 ->
+// 1.36, 96^3 5.36 -> 3.70, 128^3 4.29 -> 3.34.  The gain shrinks with the rows, and larger hierarchies,
+// not measured, keep the launches with their four times as many threads per SM.
 template <typename V>
 int setup_mg_group(scdat_ctx* ctx, const HostMg& hmg, MgGroupPlan<V>& plan, const V* cinv)
 {

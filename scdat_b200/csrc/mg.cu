@@ -2,7 +2,7 @@
 // kernels: every level's sweeps are CSR row loops (one thread per row, as the Jacobi-PCG SpMV),
 // the transfers are the <= 8-entry rows of P and the <= 27-entry rows of P^T, the coarsest
 // solve is a warp-per-row dense mat-vec held in L2.  FP32 (inner solve of the mixed form) or
-// FP64 (the plain FP64 form).  Hierarchies of up to 303,104 finest rows are solved in one launch
+// FP64 (the plain FP64 form).  Hierarchies of up to 2,424,832 finest rows are solved in one launch
 // instead (mg_group.cu).
 #include "field_kern.cuh"
 #include "mg.cuh"

@@ -17,7 +17,8 @@ namespace scdat {
 namespace {
 
 // The column of a filling entry is the row's last one, in cache beside it: with column 0 in all of
-// them the finest prolongation, most of whose rows are short, took 18 us on that one line, not 10.
+// them the finest prolongation, most of whose rows are short, took 18 us on that one line (field
+// solve at 64^3 cells 1.52 ms, not 1.43).
 template <typename S, typename V>
 __global__ void k_csr_to_ell(int R, int width, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
                              const S* __restrict__ val, V* __restrict__ ev, int32_t* __restrict__ ec)

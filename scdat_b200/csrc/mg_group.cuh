@@ -9,7 +9,7 @@
 namespace scdat {
 
 constexpr int kMgGroupThreads = 512;
-constexpr int kMgGroupRows = 4;   // rows a thread of the finest level has, at most
+constexpr int kMgGroupRows = 32;  // rows a thread of the finest level has, at most
 constexpr int kMgEllBatch = 14;   // entries of a row whose loads are in flight together
 constexpr int kMgEllMax = 42;     // most entries of an operator or restriction row
 constexpr int kMgEllTransfer = 8; // entries of a prolongation row (trilinear: 8 at most)

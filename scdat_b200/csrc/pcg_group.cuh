@@ -3,12 +3,12 @@
 // iteration.  Used by the single-context solves, the CSR entry points (pcg_group.cu) and, one
 // group per scenario, by the batched step (batch_field.cu).
 //
-// What bounds it: the two barriers of an iteration (3.4 us of 5 at 137 blocks) and the gathers'
+// What bounds it: the two barriers of an iteration (3.4 us of 5.4 at 137 blocks) and the gathers'
 // round trip to L2, not bandwidth.  The systems it takes (up to kCgMaxThreads * kCgRowsPerThread
 // rows per SM, 303,104 in all) fit the chip, so the two launches per iteration of the bandwidth
 // kernels (field_kern.cuh) were launch gaps and reduction tails, plus a host read every 16
 // iterations.  Whole field stages, two launches per iteration against one launch: FP64 33x27x41
-// cells 2.26 -> 0.77 ms, 48^3 3.6 -> 1.45, 66^3 7.05 -> 3.55; mixed 40^3 3.3 -> 1.5, 66^3 9.4 -> 5.8.
+// cells 2.14 -> 0.56 ms, 48^3 3.28 -> 1.00, 66^3 6.40 -> 2.61; mixed 40^3 3.27 -> 1.08, 66^3 7.80 -> 3.84.
 // Larger systems keep the bandwidth kernels: their rows would no longer fit registers.
 //
 // The arithmetic is that of field_kern.cuh: FP64 sums and scalars, vectors rounded to V.  Each
@@ -432,8 +432,8 @@ __device__ __forceinline__ void cg_solve_mixed(CgGroup g, const PoissonView& P, 
 
 // Launch shape for groups of the given row counts on nsm SMs: one block per SM at most, as many as
 // the rows fill (a row more per thread costs an iteration 0.8 to 1.6 us, 102 more blocks 1 us of
-// barrier: 33x27x41 cells, 35k rows, 137 blocks of 256 777 us, 69 of 512 833, 35 of 512 with two
-// rows a thread 955), then more rows per thread, the same for every group (a batch of 8 with one row
+// barrier: 33x27x41 cells, 35k rows, first barrier form, 137 blocks of 256 777 us, 69 of 512 833, 35
+// of 512 with two rows a thread 955), then more rows per thread, the same for every group (a batch of 8 with one row
 // a thread in its largest scenario and more in the others 7.33 ms, two in each 7.07); up to 512 rows one
 // block, whose barriers stay in the SM (FP64 field stage of 335 rows 151 -> 108 us, 504 rows 153 -> 127;
 // 992 rows two a thread in one block 199, in four blocks 177); !ok when that does not fit.

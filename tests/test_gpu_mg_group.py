@@ -11,9 +11,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("cells", [(16, 12, 8), (24, 16, 40), (72, 64, 64), (80, 64, 64)])
 def test_one_launch_solve_on_uneven_boxes(lib, cells):
-    """The hierarchies the one-launch solve takes (uneven boxes, a body off the lattice's even points,
-    up to 303,104 finest rows: 72 x 64 x 64 cells) and the first size of the launched passes: in both
-    forms the Jacobi-CG solution to the bars of the test above."""
+    """The hierarchies the one-launch solve takes: uneven boxes, a body off the lattice's even points,
+    fewer rows than threads and up to five rows a thread.  In both forms the Jacobi-CG solution to the
+    bars of the other multigrid tests."""
     n = np.array(cells)
     lo = n // 3
     mesh = O.kuhn_box(cells, 0.05, body=tuple((int(a), int(a) + max(2, int(b) // 5)) for a, b in zip(lo, n)), bias=-10.0)
