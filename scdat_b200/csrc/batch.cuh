@@ -97,9 +97,11 @@ void launch_batch_refresh_trec(const FieldJob* jobs, const BlockMap& tets, cudaS
 void launch_batch_zero(const FieldJob* jobs, const PushJob* pjobs, int njobs, int npjobs, int grid, cudaStream_t st);
 void launch_batch_surface(const FieldJob* jobs, int njobs, cudaStream_t st);
 void launch_batch_finalize_rhs(const FieldJob* jobs, const BlockMap& nodes, const BlockMap& rows, cudaStream_t st);
-void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const BlockMap& rows, int njobs, cudaStream_t st);
-// the mixed solve of all scenarios as one launch, when cg_plan found room for their groups
-cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const CgPlan& plan, cudaStream_t st);
+void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const CgPlan& plan, int njobs, cudaStream_t st);
+// the mixed solve of all scenarios as one launch, when cg_plan found room for their groups (rows: the
+// blocks the loops below would take)
+cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const BlockMap& rows, const CgPlan& plan,
+                               cudaStream_t st);
 // otherwise as two nested loops of launches:
 void launch_batch_outer_begin(const FieldJob* jobs, const BlockMap& rows, int njobs, unsigned long long cond_inner,
                               int* any_out, cudaStream_t st);

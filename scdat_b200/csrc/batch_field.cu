@@ -87,11 +87,11 @@ __global__ void k_batch_rhs(const FieldJob* __restrict__ jobs, BlockMap m)
 }
 
 // one block per scenario: a fresh refinement loop, and zero barrier slots for the one-launch solve
-__global__ void k_batch_prologue(const FieldJob* __restrict__ jobs)
+__global__ void k_batch_prologue(const FieldJob* __restrict__ jobs, int slot_words)
 {
     const int k = blockIdx.x;
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(jobs[k].part);
-    for (size_t i = threadIdx.x; i < kCgSlotBytes / sizeof(*slots); i += blockDim.x) slots[i] = 0ull;
+    for (int i = threadIdx.x; i < slot_words; i += blockDim.x) slots[i] = 0ull;
     if (threadIdx.x == 0) {
         PcgScalars* o = jobs[k].sco;
         o->iter = 0;
@@ -103,16 +103,18 @@ __global__ void k_batch_prologue(const FieldJob* __restrict__ jobs)
 }
 
 // The whole mixed solve of every scenario in one cooperative launch (pcg_group.cuh): the blocks
-// m gives a scenario are its group, and no group waits for another.
-template <int KR>
-__global__ void __launch_bounds__(kCgMaxThreads, 1) k_batch_solve(const FieldJob* __restrict__ jobs, BlockMap m, int smem_bytes)
+// m gives a scenario are its group, and no group waits for another; rows: the launched form's blocks.
+template <int JV, int K>
+__global__ void __launch_bounds__(kCgMaxThreads, 1)
+    k_batch_solve(const FieldJob* __restrict__ jobs, BlockMap m, BlockMap rows, int smem_bytes)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     Grid gr;
-    const FieldJob& J = jobs[map_ctx(m, gr)];
+    const int k = map_ctx(m, gr);
+    const FieldJob& J = jobs[k];
     if (J.A.R == 0) return;
-    CgGroup g{gr.b, gr.n, reinterpret_cast<unsigned long long*>(J.part)};
-    cg_solve_mixed<KR>(g, J.A, J.b, J.x, reinterpret_cast<double2*>(J.zp), J.sco, J.rtol, J.max_iter, smem, smem_bytes);
+    CgGroup g{gr.b, gr.n, reinterpret_cast<unsigned long long*>(J.part), (unsigned)(rows.first[k + 1] - rows.first[k])};
+    cg_solve_mixed<JV, K>(g, J.A, J.b, J.x, reinterpret_cast<double2*>(J.zp), J.sco, J.rtol, J.max_iter, smem, smem_bytes);
 }
 
 // FP64 residual r = b - A x and its norms into the outer scalars
@@ -277,24 +279,24 @@ void launch_batch_finalize_rhs(const FieldJob* jobs, const BlockMap& nodes, cons
     k_batch_rhs<<<rows.blocks, 256, 0, st>>>(jobs, rows);
 }
 
-void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const BlockMap&, int njobs, cudaStream_t st)
+void launch_batch_pcg_mixed_prologue(const FieldJob* jobs, const CgPlan& plan, int njobs, cudaStream_t st)
 {
-    k_batch_prologue<<<njobs, 256, 0, st>>>(jobs);
+    k_batch_prologue<<<njobs, 256, 0, st>>>(jobs, plan.ok ? (int)(plan.planes * kCgPlaneWords) : 0);
 }
 
-cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const CgPlan& plan, cudaStream_t st)
+cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, const BlockMap& rows, const CgPlan& plan,
+                               cudaStream_t st)
 {
-    auto kernel = plan.rows_per_thread == 1   ? k_batch_solve<1>
-                  : plan.rows_per_thread == 2 ? k_batch_solve<2>
-                  : plan.rows_per_thread == 3 ? k_batch_solve<3>
-                                              : k_batch_solve<4>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemBytes);
-    if (e != cudaSuccess) return e;
-    BlockMap m = groups;
+    BlockMap m = groups, r = rows;
     int smem = plan.smem;
-    void* args[] = {&jobs, &m, &smem};
-    return cudaLaunchCooperativeKernel((const void*)kernel, dim3(plan.blocks), dim3(plan.threads), args,
-                                       (size_t)plan.smem, st);
+    void* args[] = {&jobs, &m, &r, &smem};
+    return cg_dispatch(plan, [&](auto j, auto k) {
+        auto kernel = k_batch_solve<j, k>;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemBytes);
+        if (e != cudaSuccess) return e;
+        return cudaLaunchCooperativeKernel((const void*)kernel, dim3(plan.blocks), dim3(plan.threads), args,
+                                           (size_t)plan.smem, st);
+    });
 }
 
 void launch_batch_outer_begin(const FieldJob* jobs, const BlockMap& rows, int njobs, unsigned long long cond_inner,

@@ -46,12 +46,12 @@ int upload_map(MapBufs& m, const std::vector<int>& blocks, cudaStream_t st)
 }
 
 // Blocks per scenario in proportion to its share of `sizes` (at least one each).
-int build_map(MapBufs& m, const std::vector<int64_t>& sizes, int target, cudaStream_t st)
+int build_map(MapBufs& m, const std::vector<int64_t>& sizes, int target, std::vector<int>& blocks, cudaStream_t st)
 {
     const int n = (int)sizes.size();
     double tot = 0.0;
     for (int64_t v : sizes) tot += (double)std::max<int64_t>(v, 1);
-    std::vector<int> blocks((size_t)n);
+    blocks.resize((size_t)n);
     for (int k = 0; k < n; ++k) {
         int b = (int)std::floor((double)target * (double)std::max<int64_t>(sizes[k], 1) / tot + 0.5);
         blocks[k] = std::max(1, std::min(b, target));
@@ -211,12 +211,13 @@ int build_maps(scdat_batch* b)
         rr.push_back(c->pv.R);
         tt.push_back(c->hm.T);
     }
-    int rc = build_map(b->nodes, nn, b->nsm * b->tune.field_blocks_per_sm, b->st);
-    if (!rc) rc = build_map(b->rows, rr, b->nsm * b->tune.field_blocks_per_sm, b->st);
-    if (!rc) rc = build_map(b->tets, tt, b->nsm * b->tune.field_blocks_per_sm, b->st);
+    std::vector<int> grids;  // last of the rows
+    int rc = build_map(b->nodes, nn, b->nsm * b->tune.field_blocks_per_sm, grids, b->st);
+    if (!rc) rc = build_map(b->tets, tt, b->nsm * b->tune.field_blocks_per_sm, grids, b->st);
+    if (!rc) rc = build_map(b->rows, rr, b->nsm * b->tune.field_blocks_per_sm, grids, b->st);
     if (!rc) {
         std::vector<int> r(rr.begin(), rr.end()), blocks(rr.size());
-        b->solve = cg_plan(r.data(), (int)r.size(), b->nsm, blocks.data());
+        b->solve = cg_plan(r.data(), grids.data(), (int)r.size(), b->nsm, blocks.data());
         if (b->solve.ok) rc = upload_map(b->groups, blocks, b->st);
     }
     if (rc) b->err = "block map upload failed";
@@ -236,8 +237,8 @@ int enqueue_front(scdat_batch* b, cudaStream_t s)
     }
     launch_batch_surface(b->fjobs.p, nc, s);
     launch_batch_finalize_rhs(b->fjobs.p, b->nodes.view, b->rows.view, s);
-    launch_batch_pcg_mixed_prologue(b->fjobs.p, b->rows.view, nc, s);
-    if (b->solve.ok) BCK(launch_batch_solve(b->fjobs.p, b->groups.view, b->solve, s));
+    launch_batch_pcg_mixed_prologue(b->fjobs.p, b->solve, nc, s);
+    if (b->solve.ok) BCK(launch_batch_solve(b->fjobs.p, b->groups.view, b->rows.view, b->solve, s));
     return SCDAT_OK;
 }
 

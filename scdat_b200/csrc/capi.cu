@@ -417,10 +417,10 @@ int run_pcg64(scdat_ctx* ctx, const double* bvec, double* xvec, double rtol, int
         return SCDAT_OK;
     }
     int blocks;
-    const CgPlan plan = cg_plan(&A.R, 1, ctx->nsm, &blocks);
+    const CgPlan plan = cg_plan(&A.R, &ctx->grid_red, 1, ctx->nsm, &blocks);
     if (plan.ok) {
         ++ctx->launches;
-        CK(launch_cg64(plan, A, bvec, xvec, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
+        CK(launch_cg64(plan, ctx->grid_red, A, bvec, xvec, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
         PcgScalars h{};
         int rc = read_group_scalars(ctx, h);
         if (rc) return rc;
@@ -466,10 +466,10 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
     relres = 0.0;
     PcgScalars h{};
     int blocks;
-    const CgPlan plan = cg_plan(&R, 1, ctx->nsm, &blocks);
+    const CgPlan plan = cg_plan(&R, &ctx->grid_red, 1, ctx->nsm, &blocks);
     if (ctx->precond != SCDAT_PRECOND_MULTIGRID && plan.ok) {
         ++ctx->launches;
-        CK(launch_cg_mixed(plan, A, ctx->b.p, ctx->x.p, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
+        CK(launch_cg_mixed(plan, ctx->grid_red, A, ctx->b.p, ctx->x.p, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
         int rc = read_group_scalars(ctx, h);
         if (rc) return rc;
         iters = h.iter;
