@@ -121,7 +121,8 @@ struct scdat_batch {
 
 namespace {
 
-// Job tables from the contexts' current buffers (particle arrays move when a context sorts).
+// Job tables from the contexts' current buffers (particle arrays move when a context sorts).  A re-sort
+// still pending is gathered on its context's stream; the batch's stream waits for it.
 int upload_jobs(scdat_batch* b)
 {
     std::vector<PushJob> pj;
@@ -200,6 +201,10 @@ int upload_jobs(scdat_batch* b)
     b->collide = collide;
     BCK(cudaMemcpyAsync(b->pjobs.p, pj.data(), sizeof(PushJob) * pj.size(), cudaMemcpyHostToDevice, b->st));
     BCK(cudaMemcpyAsync(b->fjobs.p, fj.data(), sizeof(FieldJob) * fj.size(), cudaMemcpyHostToDevice, b->st));
+    for (scdat_ctx* c : b->ctx) {
+        BCK(cudaEventRecord(c->ev_fork, c->st));
+        BCK(cudaStreamWaitEvent(b->st, c->ev_fork, 0));
+    }
     return SCDAT_OK;
 }
 
@@ -394,11 +399,7 @@ int after_steps(scdat_batch* b, int n)
         }
     }
     if (bad) return bad;
-    if (!resorted) return SCDAT_OK;
-    // upload_jobs gathers the re-sorted stores on the contexts' streams: the next graph launch, on the
-    // batch's, waits for them
-    int rc = upload_jobs(b);
-    return rc ? rc : sync_contexts(b);
+    return resorted ? upload_jobs(b) : SCDAT_OK;
 }
 
 }  // namespace
