@@ -20,12 +20,6 @@ using namespace scdat;
 
 namespace {
 
-struct DeferBufs {
-    DBuf<uint32_t> idx[2];
-    DBuf<int> it[2];
-    DBuf<double> rem[2], vs[2];
-};
-
 struct MapBufs {
     DBuf<int> ctx_of, first;
     BlockMap view{};
@@ -140,9 +134,9 @@ int upload_jobs(scdat_batch* b)
         J.A = ChargeAcc{c->acc_l0.p + s * N, nullptr, nullptr};  // batched contexts are all mixed: one word
         J.L = c->led.p;
         J.ke_acc = c->ke_acc.p;
-        DeferBufs& d = *b->defer[j];
-        J.D1 = DeferList{b->dcount.p + 2 * j, (unsigned)d.idx[0].n, d.idx[0].p, d.it[0].p, d.rem[0].p, d.vs[0].p};
-        J.D2 = DeferList{b->dcount.p + 2 * j + 1, (unsigned)d.idx[1].n, d.idx[1].p, d.it[1].p, d.rem[1].p, d.vs[1].p};
+        BCK(b->defer[j]->grow(c->species[s].cap));  // new particles may be more than the batch was made for
+        J.D1 = b->defer[j]->list(0, b->dcount.p + 2 * j);
+        J.D2 = b->defer[j]->list(1, b->dcount.p + 2 * j + 1);
         collide = collide || draws_for_all(J.S, J.pp);
         pj.push_back(J);
     }
@@ -447,16 +441,7 @@ SCDAT_API int scdat_batch_create(int32_t n, scdat_ctx* const* ctxs, scdat_batch*
         scdat_ctx* c = b->ctx[k];
         for (int s = 0; s < (int)c->species.size(); ++s) {
             b->job_of.emplace_back(k, s);
-            auto d = std::make_unique<DeferBufs>();
-            for (int l = 0; l < 2; ++l) {
-                // pass 1 may defer a whole job; pass 2's overflow ends in pass 2
-                const size_t cap = (size_t)std::max<int64_t>(c->species[s].cap, 1) / (l ? 4 : 1) + 4096;
-                BCK(d->idx[l].alloc(cap));
-                BCK(d->it[l].alloc(cap));
-                BCK(d->rem[l].alloc(cap));
-                BCK(d->vs[l].alloc(cap));
-            }
-            b->defer.push_back(std::move(d));
+            b->defer.push_back(std::make_unique<DeferBufs>());
         }
     }
     BCK(b->dcount.alloc(2 * (size_t)njobs));

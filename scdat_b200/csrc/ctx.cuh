@@ -121,23 +121,18 @@ struct StageEvents {
     }
 };
 
-// Deferred-particle lists and counters of a chain of push passes, and the stream it runs on beside
-// the context's own (null: on that one).  The species' chains share no buffer, so that the later
-// passes of one, a few warps following long sub-step chains, run beside the first pass of the next.
-struct PushLane {
-    cudaStream_t st = nullptr;
-    DBuf<unsigned> count;  // defer-list counts [0, 1] and the three passes' work counters [2, 5)
+// Deferred-particle lists of a chain of push passes.
+struct DeferBufs {
     DBuf<uint32_t> idx[2];
     DBuf<int> it[2];
     DBuf<double> rem[2], vs[2];
     unsigned cap[2] = {0, 0};
 
-    // pass 1's list holds the largest species (it may defer every particle), pass 2's a quarter of
+    // pass 1's list holds the whole species (it may defer every particle), pass 2's a quarter of
     // it (a full one only means the overflow finishes in pass 2)
     cudaError_t grow(int64_t particles)
     {
         cudaError_t e = cudaSuccess;
-        if (!count.p) e = count.alloc(kLaneCounts);
         for (int l = 0; l < 2 && e == cudaSuccess; ++l) {
             const int64_t n = (l ? particles / 4 : particles) + 4096;
             const unsigned want = n < 0x7fffffff ? (unsigned)n : 0x7fffffffu;
@@ -149,7 +144,23 @@ struct PushLane {
         }
         return e;
     }
-    DeferList list(int l) { return DeferList{count.p + l, cap[l], idx[l].p, it[l].p, rem[l].p, vs[l].p}; }
+    DeferList list(int l, unsigned* count) { return DeferList{count, cap[l], idx[l].p, it[l].p, rem[l].p, vs[l].p}; }
+};
+
+// Lists and counters of the push passes, and the stream they run on beside the context's own (null: on
+// that one).  The species' chains share no buffer, so that the later passes of one, a few warps
+// following long sub-step chains, run beside the first pass of the next.
+struct PushLane {
+    cudaStream_t st = nullptr;
+    DBuf<unsigned> count;  // defer-list counts [0, 1] and the three passes' work counters [2, 5)
+    DeferBufs defer;
+
+    cudaError_t grow(int64_t particles)
+    {
+        cudaError_t e = count.p ? cudaSuccess : count.alloc(kLaneCounts);
+        return e == cudaSuccess ? defer.grow(particles) : e;
+    }
+    DeferList list(int l) { return defer.list(l, count.p + l); }
 };
 
 // One multigrid level on the device (level 0 shares the context's Poisson arrays and only

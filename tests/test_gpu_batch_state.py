@@ -28,3 +28,28 @@ def test_step_after_a_compaction_is_bitwise_the_settled_store_s(lib):
         for d in doms:
             d[0].close()
     _equal(out[0], out[1])
+
+
+def test_a_larger_population_between_steps(lib):
+    """A context of the batch gets four times the particles, which the null collision defers whole on
+    their first push: the batch's lists grow with them.  Bitwise the context alone."""
+    from scdat_b200 import capi
+
+    out = []
+    for batched in (False, True):
+        dom, sp, _ = _scenario((10, 9, 8), 3, 2)
+        b = capi.Batch([dom]) if batched else None
+        step = b.step if batched else dom.step
+        step(1)
+        large, _, n = _scenario((10, 9, 8), 4, 16)
+        for s in range(sp):
+            p = large.get_particles(s)
+            dom.set_particles(s, p["x"], p["v"], p["tet"], p["id"])
+            dom.set_elastic(s, 1e18, 1e-19, mode=2)
+        large.close()
+        step(2)
+        out.append(_state((dom, sp, n)))
+        if b:
+            b.close()
+        dom.close()
+    _equal([out[1]], [out[0]])
