@@ -294,8 +294,7 @@ cudaError_t launch_batch_solve(const FieldJob* jobs, const BlockMap& groups, con
         auto kernel = k_batch_solve<j, k>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemBytes);
         if (e != cudaSuccess) return e;
-        return cudaLaunchCooperativeKernel((const void*)kernel, dim3(plan.blocks), dim3(plan.threads), args,
-                                           (size_t)plan.smem, st);
+        return cg_launch((const void*)kernel, plan.blocks, plan.threads, args, (size_t)plan.smem, st);
     });
 }
 

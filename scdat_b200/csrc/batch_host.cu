@@ -223,7 +223,8 @@ int build_maps(scdat_batch* b)
     return rc;
 }
 
-// The step as launches on stream s.  With graph handles (cond_outer/cond_inner != 0) the
+// The step as launches on stream s, up to the field solve; that too when one launch does it (solve.ok
+// afterwards).  With graph handles (cond_outer/cond_inner != 0) the
 // loops are conditional nodes added by the caller; without them the host drives the loops.
 int enqueue_front(scdat_batch* b, cudaStream_t s)
 {
@@ -237,7 +238,13 @@ int enqueue_front(scdat_batch* b, cudaStream_t s)
     launch_batch_surface(b->fjobs.p, nc, s);
     launch_batch_finalize_rhs(b->fjobs.p, b->nodes.view, b->rows.view, s);
     launch_batch_pcg_mixed_prologue(b->fjobs.p, b->solve, nc, s);
-    if (b->solve.ok) BCK(launch_batch_solve(b->fjobs.p, b->groups.view, b->rows.view, b->solve, s));
+    if (b->solve.ok) {
+        const cudaError_t e = launch_batch_solve(b->fjobs.p, b->groups.view, b->rows.view, b->solve, s);
+        if (cg_refused(e))
+            b->solve.ok = false;  // this step and the next ones take the loops
+        else
+            BCK(e);
+    }
     return SCDAT_OK;
 }
 

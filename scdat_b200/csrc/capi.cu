@@ -366,9 +366,13 @@ int run_mgpcg(scdat_ctx* ctx, const V* b, V* x, V* r, V* z, V* p, V* q, bool zer
     const PoissonView& A = ctx->pv;
     const MgGroupPlan<V>& group = mg_group<V>(ctx);
     if (group.blocks > 0) {
-        ctx->launches += 1;
-        CK(launch_mgpcg_group<V>(group, b, x, r, z, p, q, zero_start, rtol, max_iter, ctx->sc.p, ctx->part.p, ctx->st));
-        return read_group_scalars(ctx, h);
+        const cudaError_t e = launch_mgpcg_group<V>(group, b, x, r, z, p, q, zero_start, rtol, max_iter, ctx->sc.p,
+                                                    ctx->part.p, ctx->st);
+        if (!cg_refused(e)) {
+            CK(e);
+            ctx->launches += 1;
+            return read_group_scalars(ctx, h);
+        }
     }
     if (zero_start) CK(cudaMemsetAsync(x, 0, sizeof(V) * A.R, ctx->st));
     int rc = pcg_scalars_init(ctx, rtol, max_iter, 0.0);
@@ -418,9 +422,11 @@ int run_pcg64(scdat_ctx* ctx, const double* bvec, double* xvec, double rtol, int
     }
     int blocks;
     const CgPlan plan = cg_plan(&A.R, &ctx->grid_red, 1, ctx->nsm, &blocks);
-    if (plan.ok) {
+    cudaError_t e = cudaErrorNotSupported;
+    if (plan.ok) e = launch_cg64(plan, ctx->grid_red, A, bvec, xvec, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st);
+    if (!cg_refused(e)) {
+        CK(e);
         ++ctx->launches;
-        CK(launch_cg64(plan, ctx->grid_red, A, bvec, xvec, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
         PcgScalars h{};
         int rc = read_group_scalars(ctx, h);
         if (rc) return rc;
@@ -467,9 +473,13 @@ int run_pcg_mixed(scdat_ctx* ctx, double rtol, int max_iter, int& iters, double&
     PcgScalars h{};
     int blocks;
     const CgPlan plan = cg_plan(&R, &ctx->grid_red, 1, ctx->nsm, &blocks);
-    if (ctx->precond != SCDAT_PRECOND_MULTIGRID && plan.ok) {
+    cudaError_t e = cudaErrorNotSupported;
+    if (ctx->precond != SCDAT_PRECOND_MULTIGRID && plan.ok)
+        e = launch_cg_mixed(plan, ctx->grid_red, A, ctx->b.p, ctx->x.p, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter,
+                            ctx->st);
+    if (!cg_refused(e)) {
+        CK(e);
         ++ctx->launches;
-        CK(launch_cg_mixed(plan, ctx->grid_red, A, ctx->b.p, ctx->x.p, ctx->p.p, ctx->sc.p, ctx->part.p, rtol, max_iter, ctx->st));
         int rc = read_group_scalars(ctx, h);
         if (rc) return rc;
         iters = h.iter;

@@ -233,7 +233,7 @@ cudaError_t launch_mgpcg_group(const MgGroupPlan<V>& mg, const V* b, V* x, V* r,
     MgGroupPlan<V> plan = mg;
     int zs = zero_start ? 1 : 0;
     void* args[] = {&plan, &b, &x, &r, &z, &p, &q, &zs, &rtol, &max_iter, &sc, &slots};
-    return cudaLaunchCooperativeKernel((const void*)k_mgpcg_group<V>, dim3(mg.blocks), dim3(kMgGroupThreads), args, 0, st);
+    return cg_launch((const void*)k_mgpcg_group<V>, mg.blocks, kMgGroupThreads, args, 0, st);
 }
 
 template void launch_csr_to_ell<float, float>(int, int, const int32_t*, const int32_t*, const float*, float*, int32_t*, cudaStream_t);

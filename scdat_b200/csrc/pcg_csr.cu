@@ -66,9 +66,11 @@ cudaError_t pcg_csr_run(int R, const int32_t* row_ptr, const int32_t* col, const
     // second row above 151,552 rows: the same order at 60^3 cells took 2460 us, this one 2040)
     const int vgrid = nsm * 8;
     const CgPlan plan = cg_plan(&R, &vgrid, 1, nsm, &blocks);
-    if (plan.ok) {
-        // s.p and s.pn lie one behind the other: the 2 R values of the direction and z
-        if ((e = launch_cg64(plan, vgrid, A, b, x, s.p, s.sc, s.part, rtol, max_iter, st)) != cudaSuccess) return e;
+    e = cudaErrorNotSupported;
+    // s.p and s.pn lie one behind the other: the 2 R values of the direction and z
+    if (plan.ok) e = launch_cg64(plan, vgrid, A, b, x, s.p, s.sc, s.part, rtol, max_iter, st);
+    if (!cg_refused(e)) {
+        if (e != cudaSuccess) return e;
         if ((e = cudaMemcpyAsync(&h, s.sc, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         if (h.done < 0) return cudaErrorLaunchTimeout;

@@ -27,14 +27,12 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1)
     cg_solve_mixed<J, K>(g, A, b, x, zp, sc, rtol, max_iter, smem, smem_bytes);
 }
 
-// Cooperative launch: the group's blocks wait on one another, so all of them have to be resident.
 template <typename K>
 cudaError_t launch_group(K kernel, const CgPlan& plan, void** args, cudaStream_t st)
 {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchCooperativeKernel((const void*)kernel, dim3(plan.blocks), dim3(plan.threads), args,
-                                       (size_t)plan.smem, st);
+    return cg_launch((const void*)kernel, plan.blocks, plan.threads, args, (size_t)plan.smem, st);
 }
 
 }  // namespace

@@ -599,6 +599,21 @@ __device__ __forceinline__ void cg_solve_mixed(CgGroup g, const PoissonView& P, 
 // blocks_of: blocks of each group.
 CgPlan cg_plan(const int* rows, const int* grids, int n, int nsm, int* blocks_of);
 
+// The runtime refused a cooperative launch: the launched form can run instead.
+inline bool cg_refused(cudaError_t e)
+{
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported;
+}
+
+// Cooperative, since a group's blocks wait on one another and all have to be resident; a refusal is the
+// returned value only.
+inline cudaError_t cg_launch(const void* kernel, int blocks, int threads, void** args, size_t smem, cudaStream_t st)
+{
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(threads), args, smem, st);
+    if (cg_refused(e)) cudaGetLastError();
+    return e;
+}
+
 // One system: queues the solve on st.  zp: 2 R values; slots: kCgSlotBytes; grid: as for cg_plan; results
 // in sc (done < 0: a barrier wait ran out).
 cudaError_t launch_cg64(const CgPlan& plan, int grid, const PoissonView& A, const double* b, double* x, double* zp,
