@@ -115,6 +115,9 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1)
     if (J.A.R == 0) return;
     CgGroup g{gr.b, gr.n, reinterpret_cast<unsigned long long*>(J.part), (unsigned)(rows.first[k + 1] - rows.first[k])};
     cg_solve_mixed<JV, K>(g, J.A, J.b, J.x, reinterpret_cast<double2*>(J.zp), J.sco, J.rtol, J.max_iter, smem, smem_bytes);
+    // the step goes on with a void potential: the flag stays until the host has seen it, also when later
+    // steps of the call solve
+    if (g.dead && threadIdx.x == 0) atomicOr(&J.led->flags, (unsigned long long)kFlagSolveWait);
 }
 
 // FP64 residual r = b - A x and its norms into the outer scalars

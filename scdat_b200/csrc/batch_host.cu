@@ -361,13 +361,18 @@ int after_steps(scdat_batch* b, int n)
     std::vector<PcgScalars> o(b->ctx.size());
     BCK(cudaMemcpy(o.data(), b->sco.p, sizeof(PcgScalars) * o.size(), cudaMemcpyDeviceToHost));
     bool resorted = false;
-    // queued on every context before the host waits for any of them
+    int bad = SCDAT_OK;
+    const auto note = [&](scdat_ctx* c, int rc) {
+        if (rc && !bad) {
+            b->err = c->err;
+            bad = rc;
+        }
+        return rc;
+    };
+    // Every context takes the steps into account, whatever fails in another.  Queued on all of them before
+    // the host waits for any.
     for (size_t k = 0; k < b->ctx.size(); ++k) {
         scdat_ctx* c = b->ctx[k];
-        if (o[k].done < 0) {
-            b->err = "field solve: a barrier wait ran out";
-            return SCDAT_ERR_CUDA;
-        }
         c->last_pcg_iter = o[k].iter;
         c->last_pcg_rel = std::sqrt(o[k].rr / (o[k].bb > 0.0 ? o[k].bb : 1.0));
         const int64_t before = c->steps;
@@ -375,30 +380,13 @@ int after_steps(scdat_batch* b, int n)
         c->sim_time += n * c->prm.dt;
         const int si = c->prm.sort_interval;
         if (si > 0 && c->steps / si != before / si) {
-            for (int s = 0; s < (int)c->species.size(); ++s) {
-                if (!species_sorts_now(c, s)) continue;
-                int rc = do_sort(c, s);
-                if (rc) {
-                    b->err = c->err;
-                    return rc;
-                }
-            }
+            for (int s = 0; s < (int)c->species.size(); ++s)
+                if (species_sorts_now(c, s)) note(c, do_sort(c, s));
             resorted = true;
         }
-        int rc = queue_flags(c);
-        if (rc) {
-            b->err = c->err;
-            return rc;
-        }
+        note(c, queue_flags(c));
     }
-    int bad = SCDAT_OK;
-    for (scdat_ctx* c : b->ctx) {
-        int rc = finish_flags(c);
-        if (rc && !bad) {
-            b->err = c->err;
-            bad = rc;
-        }
-    }
+    for (scdat_ctx* c : b->ctx) note(c, finish_flags(c));
     if (bad) return bad;
     return resorted ? upload_jobs(b) : SCDAT_OK;
 }

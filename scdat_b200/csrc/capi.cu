@@ -210,6 +210,10 @@ int finish_flags(scdat_ctx* ctx)
         if (ctx->sorting >> s & 1u) ctx->species[s].n = ctx->pin->nact[s];
     ctx->sorting = 0;
     const unsigned long long f = ctx->pin->flags;
+    if (f & kFlagSolveWait) {
+        ctx->err = "field solve: a barrier wait ran out";
+        return SCDAT_ERR_CUDA;
+    }
     if (f & kFlagBadTet) {
         ctx->err = "device flag: invalid tet index seen";
         return SCDAT_ERR_DEVICE_FLAG;
@@ -1154,6 +1158,7 @@ static int alloc_species(scdat_ctx* ctx, int s, int64_t n)
     CK(S.id.alloc((size_t)cap));
     S.cap = cap;
     S.n = n;
+    ctx->sorting &= ~(1u << s);  // a count still to be read is the old particles'
     CK(cudaMemcpyAsync(ctx->counts.p + s, &S.n, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->st));
     // new particles: no maximum speed yet (the next push's MCC takes the direct draw)
     CK(cudaMemsetAsync(ctx->vmax.p + 2 * s, 0, 2 * sizeof(unsigned), ctx->st));

@@ -213,7 +213,8 @@ struct LedgerDev {
 enum DeviceFlag : unsigned long long {
     kFlagBadTet = 1ull << 0,
     kFlagPcgNotConverged = 1ull << 1,
-    kFlagDeferOverflow = 1ull << 2,  // a stay-first pass 1 found its deferred list full
+    kFlagDeferOverflow = 1ull << 2,  // a pass 1 found its deferred list full
+    kFlagSolveWait = 1ull << 3,      // a batched field solve gave up a barrier wait
 };
 
 struct SpeciesDev {

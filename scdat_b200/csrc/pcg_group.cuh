@@ -57,7 +57,7 @@ struct CgGroup {
     unsigned long long* slots;
     unsigned vgrid = 0;
     unsigned epoch = 0;
-    bool dead = false;  // a barrier wait ran out: every result is void
+    bool dead = false;  // a barrier wait ran out: every result is void, and this block posts nothing more
 };
 
 // A sum in a slot: two 64-bit words of 32 data bits and the barrier's number, so that a reader knows
@@ -142,7 +142,7 @@ __device__ __forceinline__ void group_sync_sum(CgGroup& g, double (&v)[NV])
             if (g.n == 1) {
 #pragma unroll
                 for (int k = 0; k < NV; ++k) psum[k][0] = s[k];
-            } else {
+            } else if (!g.dead) {
                 if (DATA) fence_acq_rel();
                 slot_post(slots + (size_t)kCgSlotWords * g.b, g.epoch, s[0], NV > 1 ? s[NV - 1] : 0.0);
             }
@@ -263,7 +263,7 @@ __device__ __forceinline__ void group_sync_dots(CgGroup& g, const double (&in)[N
         if (lane >= per)
 #pragma unroll
             for (int k = 0; k < NV; ++k) t[k] = 0.0;
-        if (g.n > 1 && lane < per) {
+        if (g.n > 1 && !g.dead && lane < per) {
             if (DATA) fence_acq_rel();
             slot_post(unit_at(g.b * per + u), g.epoch, t[0], NV > 1 ? t[NV - 1] : 0.0);
         }
@@ -513,7 +513,7 @@ __device__ __forceinline__ void cg_solve64(CgGroup g, const PoissonView& P, cons
 // run_pcg_mixed in capi.cu), all passes in this call.  sc: rr, bb, iter (inner iterations in all)
 // and outer (passes) out.
 template <int J, int K>
-__device__ __forceinline__ void cg_solve_mixed(CgGroup g, const PoissonView& P, const double* b, double* xg,
+__device__ __forceinline__ void cg_solve_mixed(CgGroup& g, const PoissonView& P, const double* b, double* xg,
                                                double2* zp, PcgScalars* sc, double rtol, int max_iter,
                                                unsigned char* smem, int smem_bytes)
 {

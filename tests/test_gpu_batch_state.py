@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from faults import faults
 from test_gpu_batch_bits import _equal, _scenario, _state
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,27 @@ def test_a_larger_population_between_steps(lib):
             b.close()
         dom.close()
     _equal([out[1]], [out[0]])
+
+
+def test_a_wait_that_runs_out_in_an_earlier_step_is_reported(lib):
+    """The first step's solve lacks a block, so the last scenario's others give up their wait (some
+    seconds) and its potential is void; the second step's solve is whole.  The call has to fail, every
+    context has to count both steps, and the batch stays failed."""
+    from scdat_b200 import capi
+
+    with faults() as flib:
+        doms = [_scenario(c, 8, 2) for c in ((6, 6, 6), (7, 8, 6), (12, 11, 10))]
+        b = capi.Batch([d[0] for d in doms], use_graph=False)
+        flib.fault_launches(0, 1)
+        with pytest.raises(capi.ScdatError, match="wait ran out"):
+            b.step(2)
+        assert flib.fault_calls() == 2
+        assert [d[0].stats()["completed_steps"] for d in doms] == [2, 2, 2]
+        with pytest.raises(capi.ScdatError, match="wait ran out"):
+            b.step(1)
+        # the others' particles are counted after the re-sort of step 2, and new ones are taken as given
+        for dom, sp, n in doms[:2]:
+            assert sum(len(dom.get_particles(s)["id"]) for s in range(sp)) <= n
+        b.close()
+        for d in doms:
+            d[0].close()
