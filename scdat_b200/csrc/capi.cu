@@ -563,7 +563,8 @@ int setup_mg_group(scdat_ctx* ctx, const HostMg& hmg, MgGroupPlan<V>& plan, cons
         for (size_t r = 0; r + 1 < ptr.size(); ++r) w = std::max(w, (int)(ptr[r + 1] - ptr[r]));
         return w;
     };
-    const auto batches = [](int w) { return (w + kMgEllBatch - 1) / kMgEllBatch * kMgEllBatch; };
+    // a batch at least: a row's loads begin before its width is looked at
+    const auto batches = [](int w) { return (std::max(w, 1) + kMgEllBatch - 1) / kMgEllBatch * kMgEllBatch; };
     std::vector<MgGroupLevel<V>> table((size_t)L);
     std::vector<std::array<int, 3>> widths((size_t)L);
     for (int l = 0; l + 1 < L; ++l) {

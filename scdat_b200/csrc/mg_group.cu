@@ -33,7 +33,7 @@ __global__ void k_csr_to_ell(int R, int width, const int32_t* __restrict__ ptr, 
 }
 
 // s + sum over row i of val * x(col), in the row's order, summed in S; B entries in flight, the next
-// ones' columns beside them.
+// ones' columns beside them.  The width is a batch at least.
 template <int B, typename S, typename V>
 __device__ __forceinline__ S ell_row(const EllDev<V>& A, int i, S s, const V* x)
 {

@@ -24,3 +24,20 @@ def test_one_launch_solve_on_uneven_boxes(lib, cells):
         assert len(levels) >= 2 and rc_j == 0 and rc_m == 0 and rel_m <= rtol and it_m <= 40
         assert rel_err(phi_m, phi_j) < 1e-11
         assert rel_err(E_m, E_j) < 1e-9
+
+
+def test_levels_without_couplings(lib):
+    """Free nodes at even coordinates only: no row of the finest operator, nor of the next, has an entry
+    beside its diagonal, so their rows are filling entries alone."""
+    n = 24
+    mesh = O.kuhn_box((n, n, n), 0.05, body=None, bias=0.0)
+    at = np.rint(mesh.xyz / 0.05).astype(int)
+    free = np.all((at % 2 == 0) & (at > 0) & (at < n), axis=1)
+    mesh.dirichlet[:] = np.where(free, 0, 1)
+    rho = _charge(mesh, 9)
+    for precision, rtol in ((0, 1e-13), (1, 1e-12)):
+        rc_j, phi_j, E_j, _, _, _ = _solve(mesh, precision, False, rtol, rho)
+        rc_m, phi_m, E_m, it_m, rel_m, levels = _solve(mesh, precision, True, rtol, rho)
+        assert [lv[0] for lv in levels] == [11**3, 11**3, 5**3] and free.sum() == 11**3
+        assert rc_j == 0 and rc_m == 0 and rel_m <= rtol
+        assert rel_err(phi_m, phi_j) < 1e-11 and rel_err(E_m, E_j) < 1e-9
