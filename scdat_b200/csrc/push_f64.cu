@@ -10,6 +10,7 @@
 // to keep warps converged, and pass 1 walks from a queue and ends the rare cases in pass 2, as in
 // push_mixed.cu.
 #include "push.cuh"
+#include "segment_cloud.h"
 
 namespace scdat {
 
@@ -83,30 +84,9 @@ __device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev
                 }
             }
         } else {
-            // LinearSegmentCloud: the points tau_k = (k + 1/2) / nseg inside the tet are those of one
-            // interval of k, whose sum is in closed form.  Its ends come from the faces' crossings
-            // and are settled by the containment test of the points next to them, so that they are
-            // the points a loop over all of them would take.
-            const auto in = [&](int k) {
-                const double tau = ((double)k + 0.5) / (double)nseg;
-                const double l[4] = {ls[0] + tau * dl[0], ls[1] + tau * dl[1], ls[2] + tau * dl[2], ls[3] + tau * dl[3]};
-                return bary_inside(l);
-            };
-            double lo = 0.0, hi = 1.0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (dl[i] == 0.0) continue;  // the point tests decide
-                const double inv = 1.0 / dl[i];
-                const double a = (-kBaryEps - ls[i]) * inv, b = (1.0 + kBaryEps - ls[i]) * inv;
-                lo = fmax(lo, fmin(a, b));
-                hi = fmin(hi, fmax(a, b));
-            }
-            int ka = max(0, (int)fmin(ceil(lo * (double)nseg - 0.5), (double)nseg));
-            int kb = min(nseg - 1, (int)fmax(floor(hi * (double)nseg - 0.5), -1.0));
-            if (ka > 0 && in(ka - 1)) --ka;
-            if (kb < nseg - 1 && in(kb + 1)) ++kb;
-            while (ka <= kb && !in(ka)) ++ka;
-            while (kb >= ka && !in(kb)) --kb;
+            // LinearSegmentCloud: the points inside the tet, whose sum is in closed form
+            const SegPoints p = seg_points(ls, dl, nseg, kBaryEps);
+            const int ka = p.first, kb = p.last;
             if (ka <= kb) {
                 const double n = (double)(kb - ka + 1);
                 const double st = 0.5 * n * (double)(ka + kb + 1) / (double)nseg;
