@@ -78,9 +78,12 @@ struct ChargeAcc {
     unsigned long long* h;   // the high word, signed
 };
 
-__device__ __forceinline__ void fx_red(const ChargeAcc& A, int node, double v)
+// rest: what the rounding of v lost (2^-10 of the charge unit at most).
+__device__ __forceinline__ void fx_red(const ChargeAcc& A, int node, double v, double rest = 0.0)
 {
-    const Fx128 m = fx_from_double(fabs(v));
+    Fx128 m = fx_from_double(fabs(v));
+    const long long r = __double2ll_rn((v < 0.0 ? -rest : rest) * 18446744073709551616.0);
+    fx_add(m, Fx128{(unsigned long long)r, r >> 63});
     const unsigned long long s = v < 0.0 ? ~0ull : 0ull;  // two's complement: (x ^ s) - s negates
     const unsigned long long a = m.lo & 0xffffffffull, b = m.lo >> 32, h = (unsigned long long)m.hi;
     if (a) atomicAdd(A.l0 + node, (a ^ s) - s);

@@ -47,7 +47,7 @@ __device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev
                                              const TetGeom& g, double sx, double sy, double sz, double ex, double ey,
                                              double ez, ChargeAcc A)
 {
-    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    TwoDouble sum[4] = {};  // the sample points' contributions, exact until the 128-bit node words take them
     bool any = false;
     const double tx = ex - sx, ty = ey - sy, tz = ez - sz;
     const double qw = S.q * S.w;
@@ -56,7 +56,7 @@ __device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev
         double lam[4];
         any = tiny ? baryg(g, sx, sy, sz, lam) : baryg(g, ex, ey, ez, lam);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[i] = qw * lam[i];
+        for (int i = 0; i < 4; ++i) sum[i].hi = seg_mul(qw, lam[i]);
     } else {
         // barycentrics are affine along the segment: lam(s + tau*tr) = lam_s + tau*dlam
         double ls[4], dl[4];
@@ -78,7 +78,7 @@ __device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev
                     if (bary_inside(l)) {
                         const double cw = (S.q * gw[q] / (double)nseg) * S.w;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) sum[i] += cw * l[i];
+                        for (int i = 0; i < 4; ++i) seg_add(sum[i], seg_mul(cw, l[i]));
                         any = true;
                     }
                 }
@@ -86,22 +86,17 @@ __device__ __forceinline__ void deposit_traj(const MeshView& M, const SpeciesDev
         } else {
             // LinearSegmentCloud: the points inside the tet, whose sum is in closed form
             const SegPoints p = seg_points(ls, dl, nseg, kBaryEps);
-            const int ka = p.first, kb = p.last;
-            if (ka <= kb) {
-                const double n = (double)(kb - ka + 1);
-                const double st = 0.5 * n * (double)(ka + kb + 1) / (double)nseg;
+            any = p.first <= p.last;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) sum[i] = S.cw_seg * (n * ls[i] + st * dl[i]);
-                any = true;
-            }
+            for (int i = 0; i < 4; ++i) sum[i] = seg_sum(ls[i], dl[i], p, nseg, S.cw_seg);
         }
     }
     if (!any) return;
     const int4 tn = rec_nodes(M, t);
-    fx_red(A, tn.x, sum[0] * pp.inv_uq);
-    fx_red(A, tn.y, sum[1] * pp.inv_uq);
-    fx_red(A, tn.z, sum[2] * pp.inv_uq);
-    fx_red(A, tn.w, sum[3] * pp.inv_uq);
+    fx_red(A, tn.x, sum[0].hi * pp.inv_uq, sum[0].lo * pp.inv_uq);
+    fx_red(A, tn.y, sum[1].hi * pp.inv_uq, sum[1].lo * pp.inv_uq);
+    fx_red(A, tn.z, sum[2].hi * pp.inv_uq, sum[2].lo * pp.inv_uq);
+    fx_red(A, tn.w, sum[3].hi * pp.inv_uq, sum[3].lo * pp.inv_uq);
 }
 
 struct FlightD {

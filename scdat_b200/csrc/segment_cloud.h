@@ -58,4 +58,40 @@ SCDAT_SEG SegPoints seg_points(const double* ls, const double* dl, int nseg, dou
     return SegPoints{a, b};
 }
 
+// A value and what its rounding lost.
+struct TwoDouble {
+    double hi, lo;
+};
+
+SCDAT_SEG double seg_mul(double a, double b)  // rounded: not contracted with what it is added to
+{
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+
+// a + v: the sum of FP64 terms without their rounding errors' loss
+SCDAT_SEG void seg_add(TwoDouble& a, double v)
+{
+    const double s = a.hi + v, z = s - a.hi;
+    a.lo += (a.hi - (s - z)) + (v - z);
+    a.hi = s;
+}
+
+// The sum of c * l(tau_k) over n points from `first`, c * (n ls + m / nseg dl) with m the sum of k + 1/2.  The
+// sample points' contributions used to be rounded one by one and added exactly; this carries what each
+// product and sum rounds away, so that it is no further from the exact sum.
+SCDAT_SEG TwoDouble seg_sum(double ls, double dl, SegPoints p, int nseg, double c)
+{
+    const double n = (double)(p.last - p.first + 1), m = 0.5 * n * (double)(p.first + p.last + 1);  // exact
+    const double inv = 1.0 / (double)nseg, t = seg_mul(m, inv), tl = fma(-t, (double)nseg, m) * inv;
+    const double a = seg_mul(n, ls), b = seg_mul(t, dl);
+    const double s = a + b, z = s - a;
+    const double e = (a - (s - z)) + (b - z) + (fma(n, ls, -a) + fma(tl, dl, fma(t, dl, -b)));
+    const double hi = seg_mul(s, c);
+    return TwoDouble{hi, fma(e, c, fma(s, c, -hi))};
+}
+
 }  // namespace scdat
