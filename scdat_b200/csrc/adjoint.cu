@@ -566,6 +566,7 @@ SCDAT_API int scdat_adjoint_window(scdat_ctx* ctx, const scdat_adjoint_request* 
     if (ctx->prm.deposit_kernel == SCDAT_DEP_GAUSS3) return fail("the adjoint covers the segment-cloud and nearest-point deposits");
     for (auto& S : ctx->species)
         if (S.mcc.enabled) return fail("switch the MCC off inside an adjoint window");
+    SpareScope spare(give_back_lane, ctx);
     const int steps = rq->steps, C = rq->checkpoint > 0 ? rq->checkpoint : 10;
     const int64_t N = ctx->hm.N;
     const int nsp = (int)ctx->species.size();

@@ -134,9 +134,15 @@ int upload_jobs(scdat_batch* b)
         J.A = ChargeAcc{c->acc_l0.p + s * N, nullptr, nullptr};  // batched contexts are all mixed: one word
         J.L = c->led.p;
         J.ke_acc = c->ke_acc.p;
-        BCK(b->defer[j]->grow(c->species[s].cap));  // new particles may be more than the batch was made for
-        J.D1 = b->defer[j]->list(0, b->dcount.p + 2 * j);
-        J.D2 = b->defer[j]->list(1, b->dcount.p + 2 * j + 1);
+        // all jobs run at once: the context's own lists serve the first species of each of its lanes
+        const bool own = s > 1 || (s == 1 && c->one_lane);
+        DeferBufs& defer = own ? *b->defer[j] : c->lane_of(s).defer;
+        if (own)
+            BCK(defer.grow(c->species[s].cap));  // new particles may be more than the batch was made for
+        else
+            b->defer[j]->release();
+        J.D1 = defer.list(0, b->dcount.p + 2 * j);
+        J.D2 = defer.list(1, b->dcount.p + 2 * j + 1);
         collide = collide || draws_for_all(J.S, J.pp);
         pj.push_back(J);
     }

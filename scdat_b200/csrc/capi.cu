@@ -225,6 +225,25 @@ int finish_flags(scdat_ctx* ctx)
     return SCDAT_OK;
 }
 
+// The species' deferred lists.  A second set of them, for the species after the first, is worth 2 to 30 %
+// of a push (do_push) but 30 bytes a particle: taken only out of ample free memory (an eighth of it), and
+// given back when an allocation of a call on the context fails.
+cudaError_t grow_one_lane(scdat_ctx* ctx, int64_t cap)
+{
+    ctx->one_lane = true;
+    ctx->lane[1].defer.release();
+    for (const SpeciesState& S : ctx->species) cap = std::max(cap, S.cap);
+    return ctx->lane[0].grow(cap);
+}
+
+bool give_back_lane(void* who)
+{
+    scdat_ctx* ctx = static_cast<scdat_ctx*>(who);
+    if (ctx->one_lane || ctx->lane[1].defer.cap[0] == 0) return false;
+    cudaStreamSynchronize(ctx->st);
+    return grow_one_lane(ctx, 0) == cudaSuccess;
+}
+
 // ---- the stages ----------------------------------------------------------------------
 int do_push(scdat_ctx* ctx, bool do_mcc)
 {
@@ -252,14 +271,14 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
     // other: FP64 8^3 cells 150 -> 107 us, mixed 37x53x29 325 -> 250, mixed 64^3 2.64 -> 2.50 ms)
     int populated = 0;
     for (const SpeciesState& Ss : ctx->species) populated += Ss.n > 0;
-    const bool fork = populated > 1;
+    const bool fork = populated > 1 && !ctx->one_lane;
     if (fork) {
         CK(cudaEventRecord(ctx->ev_fork, ctx->st));
         CK(cudaStreamWaitEvent(ctx->lane[1].st, ctx->ev_fork, 0));
     }
     for (int s = 0; s < S; ++s) {
         if (ctx->species[s].cap == 0) continue;
-        PushLane& lane = ctx->lane[s > 0];
+        PushLane& lane = ctx->lane_of(s);
         cudaStream_t st = fork && s > 0 ? lane.st : ctx->st;
         ctx->push_particles += ctx->species[s].n;
         SpeciesState& Ss = ctx->species[s];
@@ -276,7 +295,8 @@ int do_push(scdat_ctx* ctx, bool do_mcc)
         SpeciesDev sd = species_dev(ctx, s);
         // no more blocks than the species has chunks for (8 warps a block, a chunk each), but one per SM
         const int grid = (int)std::max<int64_t>(ctx->nsm, std::min<int64_t>(ctx->grid_push, (Ss.n + 255) / 256));
-        if (s > 1) CK(cudaMemsetAsync(lane.count.p, 0, kLaneCounts * sizeof(unsigned), st));  // the lane's next species
+        if (s > 1 || (s == 1 && ctx->one_lane))  // the lane's next species
+            CK(cudaMemsetAsync(lane.count.p, 0, kLaneCounts * sizeof(unsigned), st));
         const DeferList d1 = lane.list(0), d2 = lane.list(1);
         ctx->launches += 3;
         ChargeAcc acc = ctx->mixed ? ChargeAcc{ctx->acc_l0.p + s * N, nullptr, nullptr}
@@ -1138,6 +1158,23 @@ SCDAT_API int scdat_set_species(scdat_ctx* ctx, int32_t n_species, const scdat_s
     return SCDAT_OK;
 }
 
+static int alloc_lane(scdat_ctx* ctx, int s, int64_t cap)
+{
+    SpareScope none(nullptr, nullptr);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!ctx->one_lane) {
+        size_t free = 0, total = 0;
+        if (s > 0 && ctx->lane[1].defer.cap[0] < cap) CK(cudaMemGetInfo(&free, &total));
+        if (s == 0 || ctx->lane[1].defer.cap[0] >= cap || DeferBufs::bytes(cap) <= free / 8) e = ctx->lane_of(s).grow(cap);
+    }
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        e = grow_one_lane(ctx, cap);
+    }
+    CK(e);
+    return SCDAT_OK;
+}
+
 static int alloc_species(scdat_ctx* ctx, int s, int64_t n)
 {
     SpeciesState& S = ctx->species[s];
@@ -1163,7 +1200,8 @@ static int alloc_species(scdat_ctx* ctx, int s, int64_t n)
     CK(cudaMemcpyAsync(ctx->counts.p + s, &S.n, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->st));
     // new particles: no maximum speed yet (the next push's MCC takes the direct draw)
     CK(cudaMemsetAsync(ctx->vmax.p + 2 * s, 0, 2 * sizeof(unsigned), ctx->st));
-    CK(ctx->lane[s > 0].grow(cap));
+    int rc = alloc_lane(ctx, s, cap);
+    if (rc) return rc;
     // sort scratch and re-sort targets must cover the largest species (allocated here, not in
     // the first re-sort of a timed run)
     size_t need = (size_t)cap;
@@ -1194,6 +1232,7 @@ SCDAT_API int scdat_set_particles(scdat_ctx* ctx, int32_t species, int64_t n, co
     ARG(species >= 0 && species < (int)ctx->species.size(), "bad species index");
     ARG(n >= 0 && (n == 0 || (x && v)), "bad particle arrays");
     ARG(n < (int64_t)0xffffffffLL, "too many particles for 32-bit ids");
+    SpareScope spare(give_back_lane, ctx);
     int rc = alloc_species(ctx, species, n);
     if (rc) return rc;
     if (n == 0) return SCDAT_OK;
@@ -1248,6 +1287,7 @@ SCDAT_API int scdat_seed_tet_particles(scdat_ctx* ctx, int32_t species, int64_t 
     }
     const int64_t n = nt * n_per_tet;
     ARG(n < (int64_t)0xffffffffLL, "too many particles for 32-bit ids");
+    SpareScope spare(give_back_lane, ctx);
     int rc = alloc_species(ctx, species, n);
     if (rc) return rc;
     if (n == 0) return SCDAT_OK;
@@ -1505,6 +1545,7 @@ SCDAT_API int scdat_seed_box_particles(scdat_ctx* ctx, int32_t species, int32_t 
     const int64_t ncell = (int64_t)(hex.size() / 3);
     const int64_t n = ncell * n_per_cell;
     ARG(n < (int64_t)0xffffffffLL, "too many particles for 32-bit ids");
+    SpareScope spare(give_back_lane, ctx);
     int rc = alloc_species(ctx, species, n);
     if (rc) return rc;
     DBuf<int32_t> dh;
@@ -1802,6 +1843,7 @@ SCDAT_API int scdat_set_field_preconditioner(scdat_ctx* ctx, int32_t kind)
 {
     if (!ctx) return SCDAT_ERR_ARG;
     ARG(kind == SCDAT_PRECOND_JACOBI || kind == SCDAT_PRECOND_MULTIGRID, "unknown preconditioner");
+    SpareScope spare(give_back_lane, ctx);
     if (kind == SCDAT_PRECOND_MULTIGRID && ctx->mgl.empty()) {
         int rc = setup_multigrid(ctx);
         if (rc) return rc;

@@ -48,6 +48,10 @@ struct DBuf {
             scratch_trim();
             e = cudaMalloc((void**)&p, count * sizeof(T));
         }
+        while (e == cudaErrorMemoryAllocation && spare_give_back()) {
+            cudaGetLastError();
+            e = cudaMalloc((void**)&p, count * sizeof(T));
+        }
         if (e == cudaSuccess) n = count;
         return e;
     }
@@ -121,12 +125,14 @@ struct StageEvents {
     }
 };
 
-// Deferred-particle lists of a chain of push passes.
+// Deferred-particle lists of a chain of push passes, each in one allocation: the entries' times left and
+// start speeds, particle numbers and sub-steps.
 struct DeferBufs {
-    DBuf<uint32_t> idx[2];
-    DBuf<int> it[2];
-    DBuf<double> rem[2], vs[2];
+    DBuf<unsigned char> mem[2];
     unsigned cap[2] = {0, 0};
+    static constexpr size_t kEntry = 2 * sizeof(double) + sizeof(uint32_t) + sizeof(int);
+
+    static size_t bytes(int64_t particles) { return kEntry * (size_t)(particles + particles / 4 + 2 * 4096); }
 
     // pass 1's list holds the whole species (it may defer every particle), pass 2's a quarter of
     // it (a full one only means the overflow finishes in pass 2)
@@ -138,13 +144,24 @@ struct DeferBufs {
             const unsigned want = n < 0x7fffffff ? (unsigned)n : 0x7fffffffu;
             if (want <= cap[l]) continue;
             cap[l] = 0;
-            if ((e = idx[l].alloc(want)) == cudaSuccess && (e = it[l].alloc(want)) == cudaSuccess &&
-                (e = rem[l].alloc(want)) == cudaSuccess && (e = vs[l].alloc(want)) == cudaSuccess)
-                cap[l] = want;
+            if ((e = mem[l].alloc(kEntry * want)) == cudaSuccess) cap[l] = want;
         }
         return e;
     }
-    DeferList list(int l, unsigned* count) { return DeferList{count, cap[l], idx[l].p, it[l].p, rem[l].p, vs[l].p}; }
+    void release()
+    {
+        for (int l = 0; l < 2; ++l) {
+            mem[l].release();
+            cap[l] = 0;
+        }
+    }
+    DeferList list(int l, unsigned* count)
+    {
+        double* rem = reinterpret_cast<double*>(mem[l].p);
+        double* vs = rem + cap[l];
+        uint32_t* idx = reinterpret_cast<uint32_t*>(vs + cap[l]);
+        return DeferList{count, cap[l], idx, reinterpret_cast<int*>(idx + cap[l]), rem, vs};
+    }
 };
 
 // Lists and counters of the push passes, and the stream they run on beside the context's own (null: on
@@ -234,7 +251,9 @@ struct scdat_ctx {
     DBuf<int64_t> stage_nodes;  // scdat_set_node_potentials staging
     DBuf<double> stage_vals;
     PushLane lane[2];  // the push of species 0, and of the others
+    bool one_lane = false;  // no room for the second one's lists: the species take turns in the first
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    PushLane& lane_of(int s) { return lane[s > 0 && !one_lane]; }
     // surface circuit of the body faces (scdat_set_surface_circuit)
     bool surface = false;
     int see_model = 0;
@@ -298,6 +317,7 @@ PushParams push_params(const scdat_ctx* ctx, bool do_mcc);
 int queue_flags(scdat_ctx* ctx);   // queues the read of the device flags and of the re-sorts' new counts
 int finish_flags(scdat_ctx* ctx);  // waits for it, takes the counts over and tests the flags
 int do_sort(scdat_ctx* ctx, int s);  // queued; finish_flags brings the host's count up to date
+bool give_back_lane(void* ctx);  // frees the second species' deferred lists (for a SpareScope)
 int do_push(scdat_ctx* ctx, bool do_mcc);
 int do_surface(scdat_ctx* ctx);
 int do_solve_field(scdat_ctx* ctx);

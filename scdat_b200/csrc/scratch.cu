@@ -39,14 +39,36 @@ cudaError_t pool_of_device(cudaMemPool_t* pool)
     return cudaSuccess;
 }
 
+thread_local SpareScope* t_spare = nullptr;
+
 }  // namespace
+
+SpareScope::SpareScope(bool (*give_back)(void*), void* who) : give_back_(give_back), who_(who), outer_(t_spare)
+{
+    t_spare = this;
+}
+
+SpareScope::~SpareScope() { t_spare = outer_; }
+
+bool spare_give_back()
+{
+    SpareScope* s = t_spare;
+    if (!s || !s->give_back_) return false;
+    SpareScope none(nullptr, nullptr);  // what give_back allocates itself has nothing to fall back on
+    return s->give_back_(s->who_);
+}
 
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st)
 {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = pool_of_device(&pool);
     if (e != cudaSuccess) return e;
-    return cudaMallocFromPoolAsync(p, bytes, pool, st);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    while (e == cudaErrorMemoryAllocation && spare_give_back()) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    return e;
 }
 
 void scratch_free(void* p, cudaStream_t st) { cudaFreeAsync(p, st); }

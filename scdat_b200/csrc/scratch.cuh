@@ -18,6 +18,23 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 void scratch_free(void* p, cudaStream_t st);
 void scratch_trim();  // gives the kept memory of every device back
 
+// Memory a call on this thread can do without, given back when an allocation fails: give_back frees some
+// and returns true, or returns false.  Scopes nest; one of a null function has none to give.
+class SpareScope {
+public:
+    SpareScope(bool (*give_back)(void*), void* who);
+    ~SpareScope();
+    SpareScope(const SpareScope&) = delete;
+    SpareScope& operator=(const SpareScope&) = delete;
+
+private:
+    bool (*give_back_)(void*);
+    void* who_;
+    SpareScope* outer_;
+    friend bool spare_give_back();
+};
+bool spare_give_back();
+
 // A scratch buffer of n values on one stream.
 template <typename T>
 struct SBuf {

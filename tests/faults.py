@@ -1,5 +1,5 @@
 """The library with launches and allocations that fail on request (cpp/launch_faults.cpp): the objects of
-the build linked once more, with the two CUDA calls wrapped."""
+the build linked once more, with some CUDA calls wrapped."""
 import contextlib
 import ctypes as C
 import os
@@ -17,7 +17,7 @@ def faulty_library():
     objs = [os.path.join(build.BUILD, s + ".o") for s in build.SOURCES]
     if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(map(os.path.getmtime, objs + [src])):
         subprocess.run([build.NVCC, *build.ARCH, "-shared", "-Xcompiler", "-fPIC", src, *objs, "-o", LIB, "-Xlinker",
-                        "--wrap=cudaLaunchCooperativeKernel,--wrap=cudaMalloc"], check=True)
+                        "--wrap=cudaLaunchCooperativeKernel,--wrap=cudaMalloc,--wrap=cudaFree,--wrap=cudaMemGetInfo"], check=True)
     return LIB
 
 
@@ -28,9 +28,10 @@ def faults():
     capi.LIB_PATH, capi._LIB = faulty_library(), None
     try:
         lib = capi.load()
-        lib.fault_alloc_above.argtypes = [C.c_size_t]
+        lib.fault_budget.argtypes = [C.c_size_t]
+        lib.fault_used.restype = C.c_size_t
         yield lib
         lib.fault_launches(0, 0)
-        lib.fault_alloc_above(0)
+        lib.fault_budget(0)
     finally:
         capi.LIB_PATH, capi._LIB = kept
