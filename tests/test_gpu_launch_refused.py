@@ -57,6 +57,14 @@ def test_multigrid_field_solve(lib, cells, precision, rtol):
     assert rel_err(one[1], launched[1]) < 1e-11 and rel_err(one[2], launched[2]) < 1e-9
 
 
+def test_multigrid_with_eleven_rows_a_thread(lib):
+    mesh = O.kuhn_box((112, 96, 80), 0.05, body=((40, 52), (30, 44), (20, 40)), bias=-10.0)
+    rho = _charge(mesh, 9)
+    one, launched = _both(lambda lib: _solve(mesh, 1, True, 1e-12, rho))
+    assert one[0] == launched[0] == 0 and abs(one[3] - launched[3]) <= 2
+    assert rel_err(one[1], launched[1]) < 1e-11 and rel_err(one[2], launched[2]) < 1e-9
+
+
 @pytest.mark.parametrize("use_graph", (True, False))
 @pytest.mark.parametrize("blocks,second", ((8, (40, 38, 39)), (2, (40, 38, 39)), (1, (40, 38, 39)), (1, (44, 42, 43))))
 def test_batch(lib, use_graph, blocks, second):
