@@ -30,8 +30,10 @@ def faults():
         lib = capi.load()
         lib.fault_budget.argtypes = [C.c_size_t]
         lib.fault_used.restype = C.c_size_t
-        yield lib
-        lib.fault_launches(0, 0)
-        lib.fault_budget(0)
+        try:
+            yield lib
+        finally:
+            lib.fault_launches(0, 0)
+            lib.fault_budget(0)
     finally:
         capi.LIB_PATH, capi._LIB = kept
