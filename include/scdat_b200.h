@@ -334,7 +334,9 @@ SCDAT_API int scdat_get_statistics(scdat_ctx* ctx, scdat_stats* st);
  * all (scenario, species) pairs, the field solve one launch over all scenarios with per-scenario
  * convergence (one per kernel, in loops on the device, when the scenarios' rows do not fit the
  * SMs at once), and the whole step is captured once as a CUDA graph.  The contexts stay valid for
- * every query (scdat_get_*); step them only through the batch while it exists. */
+ * every query (scdat_get_*) and may get new particles between steps; step them only through the
+ * batch while it exists.  SCDAT_ERR_CUDA with "a barrier wait ran out": a scenario's potential is
+ * void since some step of that call, and later calls report it again. */
 typedef struct scdat_batch scdat_batch;
 typedef struct {
     int32_t push_blocks_per_sm;   /* grid of the push launches, in blocks of 256 per SM (default 4) */

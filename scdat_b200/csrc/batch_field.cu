@@ -23,8 +23,8 @@ __device__ __forceinline__ void set_cond(unsigned long long h, unsigned v)
     if (h) cudaGraphSetConditional((cudaGraphConditionalHandle)h, v);
 }
 
-// Zero the per-step accumulators of every scenario: charge limbs, per-block kinetic-energy
-// partials, the active count and the defer-list counts.
+// Zero the per-step accumulators of every scenario: charge words, kinetic energy, total charge, the
+// active count and the defer-list counts.
 __global__ void k_batch_zero(const FieldJob* __restrict__ jobs, const PushJob* __restrict__ pjobs, int npjobs)
 {
     const FieldJob& J = jobs[blockIdx.y];

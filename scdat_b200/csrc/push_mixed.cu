@@ -929,7 +929,8 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed_batch_first(const PushJob
     }
 }
 
-// Pass 2 or 3 of every job: units are single chunks of the jobs' defer lists.
+// Pass 2 or 3 of every job: units are chunks of 32 of the jobs' defer lists, or, when one round of warps
+// takes all lists, pre[njobs + 1] entries each.
 template <int PASS>
 __global__ void __launch_bounds__(256, 4) k_push_mixed_batch(const PushJob* __restrict__ jobs, int njobs,
                                                           const int64_t* __restrict__ pre, unsigned* __restrict__ ctr)
