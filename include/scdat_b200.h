@@ -151,7 +151,9 @@ SCDAT_API int scdat_set_species(scdat_ctx* ctx, int32_t n_species, const scdat_s
 
 /* ParticleContainer::addParticles (ParticleManager.h:77) for one species.  tet_hint
  * (nullable) seeds PICCycle::addParticleLocation (PICCycle.h:71); ids (nullable) key the
- * MCC random streams (default: running index).  Replaces the species' particles. */
+ * MCC random streams (default: running index).  Replaces the species' particles.  Beside the
+ * particles, the push's lists take 30 bytes for each of the largest species, and as much again for
+ * the largest of the species after the first where that is at most an eighth of the free memory. */
 SCDAT_API int scdat_set_particles(scdat_ctx* ctx, int32_t species, int64_t n, const double* x, const double* v,
                                   const int32_t* tet_hint, const uint32_t* ids);
 

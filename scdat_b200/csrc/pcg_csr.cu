@@ -63,7 +63,7 @@ cudaError_t pcg_csr_run(int R, const int32_t* row_ptr, const int32_t* col, const
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     // the dots' order of a context's field solve (the launches below, of half the blocks, give a thread a
-    // second row above 151,552 rows: the same order at 60^3 cells took 2460 us, this one 2040)
+    // second row above 151,552 rows: their order at 60^3 cells took 2460 us, this one 1900)
     const int vgrid = nsm * 8;
     const CgPlan plan = cg_plan(&R, &vgrid, 1, nsm, &blocks);
     e = cudaErrorNotSupported;
